@@ -112,11 +112,12 @@ typedef struct wcfd_system {
 /* Krylov workspace (caller-allocated, see wcfd_krylov_workspace_floats) */
 typedef struct wcfd_krylov_ws {
     float*    vec;        /* wcfd_krylov_workspace_floats(C, ncomp) floats            */
-    double*   partials;   /* 8 * WCFD_MAX_BLOCKS doubles (reduction partials), 16-byte aligned */
+    double*   partials;   /* 8 * WCFD_MAX_BLOCKS doubles, 16-byte aligned: the grid barrier's
+                             counter, error word and the blocks' sums; every solve call
+                             zeroes what it uses first                                */
     double*   results;    /* unused, may be NULL                                      */
-    uint32_t* barrier;    /* WCFD_BARRIER_WORDS words: [WCFD_MAX_BLOCKS] the error word,
-                             [WCFD_MAX_BLOCKS + 2] the grid barrier's arrival counter
-                             (the rest unused); every solve call zeroes them first   */
+    uint32_t* barrier;    /* WCFD_BARRIER_WORDS words (not written by this version, may not be
+                             NULL)                                                    */
 } wcfd_krylov_ws;
 
 typedef struct wcfd_solve_stats {

@@ -57,6 +57,14 @@ int check_mesh(const wcfd_mesh* m) {
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// The grid's meeting state at the start of a caller's partials array (8 * WCFD_MAX_BLOCKS
+// doubles, 16-byte aligned)
+static_assert(kGridCtlBytes <= 8 * WCFD_MAX_BLOCKS * sizeof(double), "the meeting state fits the partials array");
+GridCtl grid_ctl(double* partials) {
+    char* p = reinterpret_cast<char*>(partials);
+    return GridCtl{reinterpret_cast<unsigned*>(p), reinterpret_cast<int*>(p + 128), p + 256};
+}
+
 // co-resident blocks of a cooperative kernel on the current device (cached per kernel
 // and device)
 int coop_capacity(const void* fn, int /*unused*/) {
@@ -73,8 +81,7 @@ int coop_capacity(const void* fn, int /*unused*/) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSolverBlock, 0);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int cap = per_sm * sms;
-    if (cap > WCFD_MAX_BLOCKS) cap = WCFD_MAX_BLOCKS;
-    if (cap > kSolverBlock) cap = kSolverBlock;  // grid_sync: one waiting thread per block
+    if (cap > kMaxGrid) cap = kMaxGrid;  // grid_reduce: one word per block and sum
     if (n < 64) cache[n++] = Entry{fn, dev, cap};
     return cap;
 }
@@ -115,7 +122,7 @@ int launch_krylov(const void* fn, int slot, const wcfd_mesh* m, wcfd_system A, f
     RET_IF(!fn, WCFD_ERR_ARGUMENT, "no solver kernel for this off-diagonal width");
     RET_IF(!A.diag || !A.off || !A.rhs || !x || !ws.vec || !ws.partials || !ws.barrier || !stats,
            WCFD_ERR_ARGUMENT, "null solver argument");
-    // the grid barrier stores each block's partial sums as one float4
+    // 16-byte words of the grid barrier
     RET_IF(reinterpret_cast<uintptr_t>(ws.partials) % 16 != 0, WCFD_ERR_ARGUMENT,
            "Krylov workspace: partials must be 16-byte aligned");
     RET_IF(maxiter < 0 || !(atol >= 0.0), WCFD_ERR_ARGUMENT, "bad atol or maxiter");
@@ -125,16 +132,14 @@ int launch_krylov(const void* fn, int slot, const wcfd_mesh* m, wcfd_system A, f
     long long want = (m->n_cells + WCFD_GRID_ROWS_PER_BLOCK - 1) / WCFD_GRID_ROWS_PER_BLOCK;
     int grid = (int)(want < cap ? want : cap);
     if (grid < 1) grid = 1;
-    if (cudaMemsetAsync(ws.barrier, 0, WCFD_BARRIER_WORDS * sizeof(uint32_t), st) != cudaSuccess)
+    if (cudaMemsetAsync(ws.partials, 0, kGridCtlBytes, st) != cudaSuccess)
         return set_error(WCFD_ERR_CUDA, "barrier reset failed");
     KrylovArgs a = {};
     a.m = *m;
     a.A = A;
     a.x = x;
     a.ws = ws.vec;
-    a.g.partials = ws.partials;
-    a.g.flags = ws.barrier;
-    a.g.err = reinterpret_cast<int*>(ws.barrier + WCFD_MAX_BLOCKS);
+    a.g = grid_ctl(ws.partials);
     a.atol2 = atol * atol;
     a.rtol2 = rtol * rtol;
     a.maxiter = maxiter;
@@ -281,23 +286,18 @@ int wcfd_grid_barrier_check(int32_t skip_block, int32_t phases, int32_t* result,
     LAUNCH_CHECK("occupancy query");
     RET_IF(cap <= 0, WCFD_ERR_CUDA, "barrier check kernel cannot be resident");
     RET_IF(skip_block >= cap, WCFD_ERR_ARGUMENT, "skip_block beyond the grid");
-    unsigned* words = nullptr;
-    double* partials = nullptr;
+    double* words = nullptr;
     int* bad = nullptr;
     int rc = WCFD_OK;
-    if (cudaMalloc(&words, WCFD_BARRIER_WORDS * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&partials, 8 * WCFD_MAX_BLOCKS * sizeof(double)) != cudaSuccess ||
+    if (cudaMalloc(&words, kGridCtlBytes) != cudaSuccess ||
         cudaMalloc(&bad, sizeof(int)) != cudaSuccess) {
         rc = set_error(WCFD_ERR_CUDA, "barrier check: allocation failed");
     }
-    if (rc == WCFD_OK && (cudaMemsetAsync(words, 0, WCFD_BARRIER_WORDS * sizeof(unsigned), st) != cudaSuccess ||
+    if (rc == WCFD_OK && (cudaMemsetAsync(words, 0, kGridCtlBytes, st) != cudaSuccess ||
                           cudaMemsetAsync(bad, 0, sizeof(int), st) != cudaSuccess))
         rc = set_error(WCFD_ERR_CUDA, "barrier check: memset failed");
     if (rc == WCFD_OK) {
-        GridCtl g;
-        g.partials = partials;
-        g.flags = words;
-        g.err = reinterpret_cast<int*>(words + WCFD_MAX_BLOCKS);
+        GridCtl g = grid_ctl(words);
         int skip = skip_block, ph = phases;
         void* args[] = {&g, &skip, &ph, &bad};
         int host[2] = {0, 0};
@@ -314,7 +314,6 @@ int wcfd_grid_barrier_check(int32_t skip_block, int32_t phases, int32_t* result,
         }
     }
     cudaFree(words);
-    cudaFree(partials);
     cudaFree(bad);
     return rc;
 }

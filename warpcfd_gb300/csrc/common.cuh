@@ -34,9 +34,6 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -187,97 +184,156 @@ __device__ __forceinline__ void block_reduce_ff(ff (&v)[NV]) {
     __syncthreads();
 }
 
-// Grid-wide synchronisation state living in caller-provided global memory.
-//   flags[WCFD_MAX_BLOCKS + 2]  arrival counter (zeroed before each launch)
-//   partials   [2 phase parities][2 float4 slots][WCFD_MAX_BLOCKS] per-block float-float
-//              totals, two values (hi, lo, hi, lo) per float4
+// Grid-wide synchronisation state living in caller-provided global memory (all of it zeroed
+// before each launch): an arrival counter, the error word (WCFD_OK or WCFD_BARRIER_TIMEOUT)
+// and [2 phase parities][2 sums][kMaxGrid] 16-byte words, one per block and sum: the block's
+// float-float total and the phase it belongs to.
 struct GridCtl {
-    double* partials;
-    unsigned* flags;
+    unsigned* ctr;
     int* err;
+    char* words;
 };
+
+// most blocks of a cooperative launch that meets at grid_reduce (one per SM)
+constexpr int kMaxGrid = 160;
+constexpr size_t kGridCtlBytes = 256 + 2 * 2 * (size_t)kMaxGrid * 16;
 
 __device__ __forceinline__ void red_release_add(unsigned* p, unsigned v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// 16-byte words that are loaded and stored whole
+__device__ __forceinline__ void ld_relaxed128(const void* p, unsigned long long& a, unsigned long long& b) {
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(a), "=l"(b)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void st_relaxed128(void* p, unsigned long long a, unsigned long long b) {
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], t;\n\t}" ::"l"(a),
+                 "l"(b), "l"(p)
+                 : "memory");
+}
+
+// pairwise sum of N float-float values (a tree, so that the merges overlap), result in v[0]
+template <int N>
+__device__ __forceinline__ void ff_tree(ff (&v)[N]) {
+#pragma unroll
+    for (int d = 1; d < N; d *= 2)
+#pragma unroll
+        for (int k = 0; k + d < N; k += 2 * d) ff_merge(v[k], v[k + d]);
+}
 
 // Barrier + reduction over all blocks of a cooperative launch, for phase number `phase`
-// (1, 2, 3, ... in every block).  v[] holds this block's float-float totals (from
-// block_reduce_ff); on return out[] holds the grid-wide sums (normalised float-float).
+// (1, 2, 3, ... in every block).  acc[] holds each thread's float-float sums; fin(sums) is
+// called by all lanes of warp 0 with the sums over the whole grid (normalised; the same bits
+// in every block on every run) and may write what the block needs to shared memory: a block
+// barrier follows.  sbuf: shared memory of NV * BS/2 ff.
 //
-// Thread 0 of every block stores the block's totals (two values per float4), then adds
-// one to a single arrival counter with a release reduction and waits (acquire loads) for
-// the counter to reach phase x gridDim.x.  Then warp 0 of every block reads all blocks'
-// totals and merges them in the same fixed order (lane-strided over blocks, then a
-// butterfly), so every block holds the same bits on every run without a second hop.
-// Measured on GB300 (2,000 barriers of two sums, cooperative launch): 2.47 us per barrier
-// at 152 blocks, against 3.4 us for an aggregator barrier (per-block flags, block 0
-// merging and releasing a `done` word) and 1.26 us for the counter alone.  The all-read
-// cost grows with the number of blocks (4.7 us at 456: every block requests the same
-// lines), so the Krylov kernels run one 1,024-thread block per SM.  Totals are double-
-// buffered by phase parity: a buffer is rewritten only after every block has passed the
-// phase that read it.  The wait is bounded: on timeout the block sets *err and returns
-// false.  NV <= 4.
-template <int NV, int BS>
-__device__ bool grid_sync(const GridCtl& g, const ff* v, ff* out, unsigned phase) {
-    static_assert(NV >= 1 && NV <= 4, "grid_sync carries 1..4 sums");
-    constexpr int NQ = (NV + 1) / 2;
+// The block stage: one butterfly level in every warp, then BS/2 values in shared memory, of
+// which warp i merges sum i (BS/64 per lane as a tree, then a butterfly) and stores it as one
+// 16-byte word that carries its phase.  Beside it, from the same block barrier on, warp NV
+// publishes everything the block wrote so far: a release reduction on the arrival counter,
+// whose fence (about 750 cycles) so overlaps the merging (about 580).  Warp 0 waits for the
+// counter (acquire), then reads every block's word and merges them in one fixed order.  A
+// word that is still on its way shows an older phase and is read again; words are
+// double-buffered by phase parity (a block stores phase k+2 only after every block has
+// arrived at k+1, and so has read k).
+// Measured (152 blocks, two sums, block stage included): 2.07 us a barrier; 3.05 us for
+// butterflies in every warp, partial sums ordered by the counter's own release and separate
+// broadcasts.  Also tried: totals polled directly instead of a counter, in 1 / 4 / 8 / 16
+// copies (6.4 / 3.9 / 3.8 / 3.5 us: 152 blocks polling 152 words), the words loaded along
+// with every poll (2.3-2.7 us), a relaxed poll with a fence after it (2.5 us).
+// Every wait is bounded: on timeout the block sets *err and returns false.  NV <= 2.
+template <int NV, int BS, typename Fin>
+__device__ __forceinline__ bool grid_reduce(const GridCtl& g, ff (&acc)[NV], ff* sbuf, unsigned phase, Fin&& fin) {
+    static_assert(NV >= 1 && NV <= 2 && BS % 64 == 0, "one or two sums");
+    constexpr int H = BS / 2;                 // values of one sum left in shared memory
+    constexpr int PER = H / 32;               // per lane of the merging warp
+    constexpr int POLL = (kMaxGrid + 31) / 32;
     __shared__ int s_fail;
-    __shared__ ff s_res[NV];
-    float4* pb = reinterpret_cast<float4*>(g.partials) + (size_t)(phase & 1u) * NQ * WCFD_MAX_BLOCKS;
-    unsigned* ctr = g.flags + WCFD_MAX_BLOCKS + 2;
-    if (threadIdx.x == 0) {
-        s_fail = 0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_fail = 0;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const ff a = v[2 * q];
-            const ff b = 2 * q + 1 < NV ? v[2 * q + 1] : ff_zero();
-            pb[q * WCFD_MAX_BLOCKS + blockIdx.x] = make_float4(a.hi, a.lo, b.hi, b.lo);
-        }
+    for (int i = 0; i < NV; ++i) {
+        ff_shfl_merge(acc[i], 16);
+        if (lane < 16) sbuf[i * H + wid * 16 + lane] = acc[i];
     }
     __syncthreads();  // every thread's writes of the phase happen before the release below
-    if (threadIdx.x == 0) {
-        red_release_add(ctr, 1u);
-        const unsigned target = phase * gridDim.x;
-        if ((int)(ld_acquire(ctr) - target) < 0) {
-            const uint64_t t0 = global_ns();
+    if (wid == NV && lane == 0) red_release_add(g.ctr, 1u);
+    if (wid < NV) {
+        char* words = g.words + (size_t)(phase & 1u) * (2 * kMaxGrid * 16);
+        ff v[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) v[k] = sbuf[wid * H + k * 32 + lane];
+        ff_tree(v);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(v[0], o);
+        if (lane == 0)
+            st_relaxed128(words + (size_t)(wid * kMaxGrid + blockIdx.x) * 16,
+                          ((unsigned long long)__float_as_uint(v[0].lo) << 32) | __float_as_uint(v[0].hi), phase);
+        if (wid == 0) {
+            const int G = (int)gridDim.x;
+            const unsigned target = phase * gridDim.x;
+            unsigned long long w[NV][POLL];
+            bool ok = true;
             unsigned spins = 0;
-            while ((int)(ld_acquire(ctr) - target) < 0) {
-                if ((++spins & 31u) == 0u && global_ns() - t0 > kBarrierTimeoutNs) {
-                    s_fail = 1;
-                    atomicExch(g.err, WCFD_BARRIER_TIMEOUT);
-                    break;
+            uint64_t t0 = 0;
+            for (;;) {
+                if ((int)(ld_acquire(g.ctr) - target) >= 0) {  // one address: the same answer in every lane
+                    unsigned long long tag[NV][POLL];
+                    bool all = true;
+#pragma unroll
+                    for (int i = 0; i < NV; ++i)
+#pragma unroll
+                        for (int k = 0; k < POLL; ++k) {
+                            const int b = k * 32 + lane;
+                            w[i][k] = 0;
+                            tag[i][k] = phase;
+                            if (b < G) ld_relaxed128(words + (size_t)(i * kMaxGrid + b) * 16, w[i][k], tag[i][k]);
+                        }
+#pragma unroll
+                    for (int i = 0; i < NV; ++i)
+#pragma unroll
+                        for (int k = 0; k < POLL; ++k) all = all && (unsigned)tag[i][k] == phase;
+                    if (__all_sync(0xffffffffu, all)) break;
+                }
+                if ((++spins & 31u) == 0u) {
+                    const uint64_t t = global_ns();
+                    if (t0 == 0) t0 = t;
+                    if (__any_sync(0xffffffffu, t - t0 > kBarrierTimeoutNs)) {
+                        ok = false;
+                        break;
+                    }
                 }
             }
-        }
-    }
-    __syncthreads();
-    if (s_fail) return false;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        ff x[2 * NQ];
+            if (!ok) {
+                if (lane == 0) {
+                    s_fail = 1;
+                    atomicExch(g.err, WCFD_BARRIER_TIMEOUT);
+                }
+            } else {
+                ff sums[NV];
 #pragma unroll
-        for (int i = 0; i < 2 * NQ; ++i) x[i] = ff_zero();
-        for (int k = lane; k < (int)gridDim.x; k += 32) {
+                for (int i = 0; i < NV; ++i) {
+                    ff x[POLL];
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const float4 t = __ldcg(pb + q * WCFD_MAX_BLOCKS + k);
-                ff_merge(x[2 * q], ff{t.x, t.y});
-                ff_merge(x[2 * q + 1], ff{t.z, t.w});
+                    for (int k = 0; k < POLL; ++k)
+                        x[k] = ff{__uint_as_float((unsigned)w[i][k]), __uint_as_float((unsigned)(w[i][k] >> 32))};
+                    ff_tree(x);
+                    sums[i] = x[0];
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < NV; ++i) ff_shfl_merge(sums[i], o);
+#pragma unroll
+                for (int i = 0; i < NV; ++i) sums[i] = ff_norm(sums[i]);
+                fin(sums);
             }
         }
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(x[i], o);
-            if (lane == 0) s_res[i] = ff_norm(x[i]);
-        }
     }
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NV; ++i) out[i] = s_res[i];
-    __syncthreads();
-    return true;
+    return !s_fail;
 }
 
 // NVTX range over a host scope (a stage of a step), for Nsight Systems timelines: one

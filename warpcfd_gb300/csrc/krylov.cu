@@ -1,6 +1,7 @@
 // Persistent Krylov solvers: one cooperative launch per solve, rows distributed
 // grid-stride over all co-resident blocks, fp64-accurate dot products (exact products
-// summed in float-float across threads, warps and blocks; common.cuh) reduced deterministically at bounded grid barriers.  They replace warp.optim.linear.cg /
+// summed in float-float across threads, warps and blocks; common.cuh) reduced deterministically
+// at bounded grid barriers.  They replace warp.optim.linear.cg /
 // bicgstab with the diagonal (Jacobi) preconditioner as called by Equation.solve_Axb
 // (warp_cfd/FV/terms/equation.py:195-200).  Stop test: ||r||_2 <= atol before an
 // iteration, or maxiter iterations.
@@ -12,7 +13,8 @@
 // needs two grid barriers instead of three and a BiCGSTAB iteration three instead of five.
 //
 // The scalar recurrences (alpha, beta, omega, the stop test) run on the float-float sums
-// in thread 0 of each block and reach the other threads through shared memory: GB300
+// in thread 0 of each block, inside the reduction (grid_reduce), and reach the other threads
+// through shared memory behind its last block barrier: GB300
 // runs fp64 at about 1/64 of its fp32 rate (a dependent fp64 division costs about 600
 // cycles), and every thread of the grid waits for these few operations.
 #include "common.cuh"
@@ -41,27 +43,23 @@ __device__ void fail_stats(const KrylovArgs& a, int k) {
     }
 }
 
-// block-reduce the float-float accumulators `acc` and sum them over the grid into the
-// float-float array `out` (NV values)
-#define SYNC(NV, acc, out)                                         \
-    do {                                                           \
-        block_reduce_ff<NV, BS>(acc);                              \
-        if (!grid_sync<NV, BS>(a.g, acc, out, ++phase)) {          \
-            fail_stats(a, sc.k);                                   \
-            return;                                                \
-        }                                                          \
+// sum the float-float accumulators `acc` over the grid; fin(sums) runs in warp 0
+// (grid_reduce, common.cuh), thread 0 of which owns the scalars that follow from them
+#define REDUCE(NV, acc, ...)                                                  \
+    do {                                                                      \
+        if (!grid_reduce<NV, BS>(a.g, acc, sbuf, ++phase, __VA_ARGS__)) {     \
+            fail_stats(a, sc.k);                                              \
+            return;                                                           \
+        }                                                                     \
     } while (0)
 
-// set-up scalars from the initial r.r and b.b; block 0 records ||r_0|| and ||b||
-__device__ void init_scalars(const KrylovArgs& a, KScalars& sc, const ff& rr, const ff& bb) {
+// set-up scalars from the initial r.r; block 0 records ||r_0||
+__device__ __forceinline__ void init_scalars(const KrylovArgs& a, KScalars& sc, const ff& rr) {
     const double rr0 = ff_to_double(rr);
     sc.rr = rr;
     sc.thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * rr0)));
     sc.go = (0 < a.maxiter && ff_gt(sc.rr, sc.thr2));
-    if (blockIdx.x == 0) {
-        a.stats->initial_residual = sqrt(rr0);
-        a.stats->rhs_norm = sqrt(ff_to_double(bb));
-    }
+    if (blockIdx.x == 0) a.stats->initial_residual = sqrt(rr0);
 }
 
 __device__ void write_stats(const KrylovArgs& a, const KScalars& sc) {
@@ -135,6 +133,7 @@ __device__ __forceinline__ int ell_column(const int* __restrict__ col, const int
 template <int W, bool kD>
 __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
     __shared__ KScalars sc;
+    __shared__ ff sbuf[2 * BS / 2];
     const int C = a.m.n_cells;
     float* r = a.ws;
     float* pbuf[2] = {a.ws + (size_t)C, a.ws + 2 * (size_t)C};
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
     }
 
     // r = b - A x ; z = M r ; p = z ; rr = r.r ; rz = r.z ; bb = b.b
-    ff acc[3] = {ff_zero(), ff_zero(), ff_zero()};
+    ff acc[2] = {ff_zero(), ff_zero()}, accb[1] = {ff_zero()};
     for (int i = i0; i < C; i += stride) {
         float ax = diag[i] * x[i];
 #pragma unroll
@@ -170,17 +169,17 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
         pbuf[0][i] = zi;
         ff_fma(acc[0], ri, ri);
         ff_fma(acc[1], ri, zi);
-        ff_fma(acc[2], b[i], b[i]);
+        ff_fma(accb[0], b[i], b[i]);
     }
-    ff red[3];
-    SYNC(3, acc, red);
-    if (threadIdx.x == 0) {
-        init_scalars(a, sc, red[0], red[2]);
-        sc.rz = red[1];
+    REDUCE(1, accb, [&](const ff* s) {
+        if (threadIdx.x == 0 && blockIdx.x == 0) a.stats->rhs_norm = sqrt(ff_to_double(s[0]));
+    });
+    REDUCE(2, acc, [&](const ff* s) {
+        if (threadIdx.x != 0) return;
+        init_scalars(a, sc, s[0]);
+        sc.rz = s[1];
         sc.bf = 0.0f;  // the first direction is z itself
-        sc.af = 0.0f;
-    }
-    __syncthreads();
+    });
     int cur = 0;
     float pending = 0.0f;  // alpha of the last completed iteration, not yet added to x
     while (sc.go) {
@@ -234,17 +233,15 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
                 ff_fma(accq[0], p2, q2);
             }
         }
-        ff pq[1];
-        SYNC(1, accq, pq);
-        if (threadIdx.x == 0) {
+        REDUCE(1, accq, [&](const ff* pq) {
+            if (threadIdx.x != 0) return;
             if (pq[0].hi == 0.0f) {
                 sc.status = WCFD_KRYLOV_BREAKDOWN;
                 sc.go = 0;
             } else {
                 sc.af = ff_div_to_float(sc.rz, pq[0]);
             }
-        }
-        __syncthreads();
+        });
         pending = 0.0f;  // alpha_prev p_old is in x now
         if (!sc.go) break;
         const float af = sc.af;
@@ -258,16 +255,14 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
             ff_fma(acc2[0], ri, ri);
             ff_fma(acc2[1], ri, zi);
         }
-        ff red2[2];
-        SYNC(2, acc2, red2);
-        if (threadIdx.x == 0) {
-            sc.rr = red2[0];
-            sc.bf = sc.rz.hi != 0.0f ? ff_div_to_float(red2[1], sc.rz) : 0.0f;
-            sc.rz = red2[1];
+        REDUCE(2, acc2, [&](const ff* s) {
+            if (threadIdx.x != 0) return;
+            sc.rr = s[0];
+            sc.bf = sc.rz.hi != 0.0f ? ff_div_to_float(s[1], sc.rz) : 0.0f;
+            sc.rz = s[1];
             sc.k += 1;
             sc.go = (sc.k < a.maxiter && ff_gt(sc.rr, sc.thr2));
-        }
-        __syncthreads();
+        });
         pending = af;
         cur ^= 1;
     }
@@ -285,6 +280,7 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
 template <int W>
 __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
     __shared__ KScalars sc;
+    __shared__ ff sbuf[2 * BS / 2];
     const int C = a.m.n_cells;
     const size_t n3 = 3 * (size_t)C;
     float* r = a.ws;
@@ -333,15 +329,14 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
             ff_fma(acc[1], b[q], b[q]);
         }
     }
-    ff red[2];
-    SYNC(2, acc, red);
-    if (threadIdx.x == 0) {
-        init_scalars(a, sc, red[0], red[1]);
-        sc.rho = red[0];
+    REDUCE(2, acc, [&](const ff* v) {
+        if (threadIdx.x != 0) return;
+        init_scalars(a, sc, v[0]);
+        sc.rho = v[0];
         sc.bf = 0.0f;  // the first direction is r itself
         sc.of = 0.0f;
-    }
-    __syncthreads();
+        if (blockIdx.x == 0) a.stats->rhs_norm = sqrt(ff_to_double(v[1]));
+    });
     int cur = 0;
     while (sc.go) {
         const float bf = sc.bf, of0 = sc.of;
@@ -379,9 +374,8 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
                 ff_fma(accv[0], r0[q], vi[o]);
             }
         }
-        ff r0v[1];
-        SYNC(1, accv, r0v);
-        if (threadIdx.x == 0) {
+        REDUCE(1, accv, [&](const ff* r0v) {
+            if (threadIdx.x != 0) return;
             if (r0v[0].hi == 0.0f) {
                 sc.status = WCFD_KRYLOV_BREAKDOWN;
                 sc.go = 0;
@@ -389,8 +383,7 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
                 sc.alpha = ff_div(sc.rho, r0v[0]);
                 sc.af = ff_to_float(sc.alpha);
             }
-        }
-        __syncthreads();
+        });
         if (!sc.go) break;
         const float af = sc.af;
         // s = r - alpha v ; x += alpha M p ; t = A (M s) ; t.t ; t.s
@@ -425,13 +418,11 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
                 ff_fma(acct[1], ti[o], si[o]);
             }
         }
-        ff ts[2];
-        SYNC(2, acct, ts);
-        if (threadIdx.x == 0) {
+        REDUCE(2, acct, [&](const ff* ts) {
+            if (threadIdx.x != 0) return;
             sc.omega = ts[0].hi != 0.0f ? ff_div(ts[1], ts[0]) : ff_zero();
             sc.of = ff_to_float(sc.omega);
-        }
-        __syncthreads();
+        });
         const float of = sc.of;
         // x += omega M s ; r = s - omega t ; r.r ; r0.r -- every load of the row issued
         // before its first store (x and r may alias the others as far as the compiler
@@ -458,9 +449,8 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
                 ff_fma(accr[1], rv0[o], ri);
             }
         }
-        ff rr2[2];
-        SYNC(2, accr, rr2);
-        if (threadIdx.x == 0) {
+        REDUCE(2, accr, [&](const ff* rr2) {
+            if (threadIdx.x != 0) return;
             sc.rr = rr2[0];
             sc.k += 1;
             if (sc.omega.hi == 0.0f || sc.rho.hi == 0.0f) {
@@ -471,8 +461,7 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
                 sc.rho = rr2[1];
                 sc.go = (sc.k < a.maxiter && ff_gt(sc.rr, sc.thr2));
             }
-        }
-        __syncthreads();
+        });
         cur ^= 1;
     }
     write_stats(a, sc);
@@ -532,16 +521,18 @@ const void* residual64_kernel_for(int W) {
 // failure made without a fault: nothing ever sets the count they wait for).
 __global__ void __launch_bounds__(BS, 1) barrier_check_kernel(GridCtl g, int skip, int phases, int* bad) {
     if ((int)blockIdx.x == skip) return;
+    __shared__ ff sbuf[2 * BS / 2];
     unsigned phase = 0;
     const float G = (float)gridDim.x;
     for (int p = 0; p < phases; ++p) {
         ff acc[2] = {ff{(float)(blockIdx.x + 1 + p), 0.0f}, ff{1.0f, 0.0f}};
-        ff out[2];
         if (threadIdx.x != 0) acc[0] = acc[1] = ff_zero();
-        if (!grid_sync<2, BS>(g, acc, out, ++phase)) return;
-        const float want0 = G * (G + 1.0f) * 0.5f + G * (float)p;  // exact below 2^24
-        if (threadIdx.x == 0 && (ff_to_double(out[0]) != (double)want0 || ff_to_double(out[1]) != (double)G))
-            atomicOr(bad, 1);
+        const bool ok = grid_reduce<2, BS>(g, acc, sbuf, ++phase, [&](const ff* s) {
+            const float want0 = G * (G + 1.0f) * 0.5f + G * (float)p;  // exact below 2^24
+            if (threadIdx.x == 0 && (ff_to_double(s[0]) != (double)want0 || ff_to_double(s[1]) != (double)G))
+                atomicOr(bad, 1);
+        });
+        if (!ok) return;
     }
 }
 
