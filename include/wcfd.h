@@ -37,6 +37,9 @@ extern "C" {
 #define WCFD_BARRIER_TIMEOUT     5  /* a grid barrier wait gave up (bounded spin)   */
 #define WCFD_ERR_TOO_LARGE       6  /* size beyond what the entry point supports    */
 
+/* marks a wcfd_mesh.slot_mask that is in use (low bits: the slots, popcount = ell_width) */
+#define WCFD_SLOT_MASK 0x57430000
+
 /* field mask bits: u, v, w, p (columns 0..3 of cell_values) */
 #define WCFD_U 1u
 #define WCFD_V 2u
@@ -55,7 +58,12 @@ typedef struct wcfd_mesh {
     int32_t n_bfaces;         /* B */
     int32_t faces_per_cell;   /* F (<= 6) */
     int32_t ell_width;        /* W (<= F) */
-    int32_t pad_;
+    int32_t slot_mask;        /* WCFD_SLOT_MASK | the cell slots that hold an off-diagonal: bit f
+                                 set = the face in slot f has its own off-diagonal slot (the
+                                 number of set bits below f), zero and with the row's own
+                                 column where that face is on the boundary.  Any other value:
+                                 a row's off-diagonals stand in slot order from slot 0 on,
+                                 its padding after them                                  */
     const int32_t* face_owner;    /* [K]   owner cell (lower id)                      */
     const int32_t* face_nbr;      /* [K]   neighbour cell, -1 on boundary faces       */
     const int32_t* face_brow;     /* [K]   row in the boundary tables, -1 internal    */
@@ -74,9 +82,9 @@ typedef struct wcfd_mesh {
                                      and 0; read only by the opt-in explicit internal terms
                                      (wcfd_params.explicit_terms), may be NULL otherwise */
     const int16_t* ell_dcol;      /* [W*C] ell_col - row as int16, when every |ell_col - row|
-                                     <= 32767 (e.g. a structured numbering), else NULL: the
-                                     grid-cooperative CG then streams 2 bytes per slot
-                                     instead of 4 (the same columns, the same bits) */
+                                     <= 32767 (e.g. a structured numbering), else NULL: where
+                                     the grid-cooperative CG reads columns it then streams 2
+                                     bytes per slot instead of 4 (the same columns and bits) */
 } wcfd_mesh;
 
 /* boundary tables, one row per boundary face, columns u,v,w,p */

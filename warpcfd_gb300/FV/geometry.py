@@ -29,7 +29,9 @@ from __future__ import annotations
 
 import numpy as np
 
+from .._lib import SLOT_MASK
 
+CLUSTER_ROWS = 65536  # most rows of a system solved by one thread-block cluster (16 x 4,096)
 NULL_SLOT = np.int32(-2**31)  # the face reference of a null slot (kNullSlot in the kernels)
 
 
@@ -105,13 +107,26 @@ def build_geometry(mesh, correction: bool = False) -> dict:
     # at least one row: a mesh without internal faces (W = 0, one cell) still hands the
     # kernels a valid array, whose padding row they never read
     ell_col = np.repeat(np.arange(C, dtype=np.int32)[None, :], max(W, 1), axis=0).copy()
-    pos = (np.cumsum(m, axis=1) - 1)
+    # The off-diagonal slot of a cell's face.  On meshes past the cluster solvers' reach (their
+    # columns live in shared memory anyway), where the cells use no more slots than the
+    # fullest of them has neighbours (every hex's +x face is slot 3, say) and neighbouring
+    # rows mostly have the same column offsets slot by slot (a structured numbering), each used
+    # face slot has its own off-diagonal slot in every row, with the padding where the boundary
+    # faces are: rows beside a boundary then have their neighbours' offsets too, and the grid CG
+    # needs no column loads.  Else the off-diagonals of a row stand from slot 0 on.
+    used = m.any(axis=0)
+    rel = nbr - np.arange(C, dtype=np.int64)[:, None]
+    both = m[1:] & m[:-1]
+    alike = int(np.count_nonzero(both & (rel[1:] == rel[:-1])))
+    in_place = C > CLUSTER_ROWS and W > 0 and int(used.sum()) == W and 2 * alike > int(np.count_nonzero(both))
+    slot_mask = SLOT_MASK | int(np.sum(used.astype(np.int64) << np.arange(F))) if in_place else 0
+    pos = np.broadcast_to(np.cumsum(used) - 1, m.shape) if in_place else np.cumsum(m, axis=1) - 1
     cc, ff = np.nonzero(m)
     ell_col[pos[cc, ff], cc] = nbr[cc, ff]
     ell_dcol = ell_offsets(ell_col) if W > 0 else None
 
     return dict(
-        n_cells=C, n_faces=K, n_bfaces=len(bids), faces_per_cell=F, ell_width=W,
+        n_cells=C, n_faces=K, n_bfaces=len(bids), faces_per_cell=F, ell_width=W, slot_mask=slot_mask,
         face_owner=P.astype(np.int32), face_nbr=N.astype(np.int32), face_brow=brow,
         face_interp=face_interp, face_normal=face_normal, face_gdiff=gdiff.astype(np.float32),
         face_rpf=rpf.astype(np.float32), cell_slot=cell_slot, cell_volume=vol.astype(np.float32),

@@ -140,7 +140,7 @@ class FVM:
                 self._gdiff_corrected = torch.from_numpy(gc).to(self.device)
             gdiff = self._gdiff_corrected
         return _lib.Mesh_t(
-            g["n_cells"], g["n_faces"], g["n_bfaces"], g["faces_per_cell"], g["ell_width"], 0,
+            g["n_cells"], g["n_faces"], g["n_bfaces"], g["faces_per_cell"], g["ell_width"], g["slot_mask"],
             g["face_owner"].data_ptr(), g["face_nbr"].data_ptr(), g["face_brow"].data_ptr(),
             g["face_interp"].data_ptr(), g["face_normal"].data_ptr(), gdiff.data_ptr(),
             g["face_rpf"].data_ptr(), g["cell_slot"].data_ptr(), g["cell_volume"].data_ptr(),

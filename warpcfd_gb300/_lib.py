@@ -26,6 +26,7 @@ WCFD_U, WCFD_V, WCFD_W, WCFD_P, WCFD_ALL = 1, 2, 4, 8, 15
 # wcfd_params.convection per ConvectionTerm interpolation scheme
 CONVECTION = {"upwind": 0, "upwindLinear": 0, "central difference": 1}
 MAX_BLOCKS = 2048
+SLOT_MASK = 0x57430000  # marks a wcfd_mesh.slot_mask in use
 BARRIER_WORDS = MAX_BLOCKS + 4
 STATS_BYTES = 32
 
@@ -41,7 +42,7 @@ vp = ct.c_void_p
 
 class Mesh_t(ct.Structure):
     _fields_ = [("n_cells", ct.c_int32), ("n_faces", ct.c_int32), ("n_bfaces", ct.c_int32),
-                ("faces_per_cell", ct.c_int32), ("ell_width", ct.c_int32), ("pad_", ct.c_int32),
+                ("faces_per_cell", ct.c_int32), ("ell_width", ct.c_int32), ("slot_mask", ct.c_int32),
                 ("face_owner", vp), ("face_nbr", vp), ("face_brow", vp), ("face_interp", vp),
                 ("face_normal", vp), ("face_gdiff", vp), ("face_rpf", vp), ("cell_slot", vp),
                 ("cell_volume", vp), ("ell_col", vp), ("boundary_face", vp), ("face_dvec", vp),

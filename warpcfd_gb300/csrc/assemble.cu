@@ -81,6 +81,7 @@ __device__ __forceinline__ void momentum_assemble_body(const wcfd_mesh& m, const
     float dx[3] = {0.0f, 0.0f, 0.0f};
     float b[3] = {0.0f, 0.0f, 0.0f};
     int j = 0;
+    const unsigned bits = slot_bits(m);
     const float4* slots = reinterpret_cast<const float4*>(m.cell_slot);
     // Every slot's face reference first, then every face's flux, neighbour and coefficient,
     // all independent loads: a thread's chain of global-memory round trips is two deep
@@ -103,6 +104,10 @@ __device__ __forceinline__ void momentum_assemble_body(const wcfd_mesh& m, const
 #pragma unroll
     for (int f = 0; f < kMaxSlots; ++f) {
         const int sk = sks[f];
+        if ((bits >> f) & 1u) {  // this face's own off-diagonal slot
+            j = __popc(bits & ((1u << f) - 1u));
+            if (sk == kNullSlot || nbs[f] < 0) sys.off[(size_t)j * C + c] = 0.0f;
+        }
         if (sk == kNullSlot) continue;
         const bool owner_side = sk >= 0;
         const int k = owner_side ? sk : ~sk;
@@ -151,7 +156,8 @@ __device__ __forceinline__ void momentum_assemble_body(const wcfd_mesh& m, const
             }
         }
     }
-    for (; j < m.ell_width; ++j) sys.off[(size_t)j * C + c] = 0.0f;
+    if (!bits)
+        for (; j < m.ell_width; ++j) sys.off[(size_t)j * C + c] = 0.0f;
     const float V = __ldg(m.cell_volume + c);
     const float4 cv = ld4(s.cell_values + 4 * (size_t)c);
     const float* gp = s.cell_gradients + 12 * (size_t)c + 9;
@@ -232,6 +238,7 @@ __device__ __forceinline__ void pressure_assemble_body(const wcfd_mesh& m, const
     const int C = m.n_cells;
     float d = 0.0f, b = 0.0f;
     int j = 0;
+    const unsigned bits = slot_bits(m);
     const bool ref = (c == prm.ref_cell);
     const float4* slots = reinterpret_cast<const float4*>(m.cell_slot);
     // the same two-deep load structure as the momentum assembly
@@ -251,6 +258,10 @@ __device__ __forceinline__ void pressure_assemble_body(const wcfd_mesh& m, const
 #pragma unroll
     for (int f = 0; f < kMaxSlots; ++f) {
         const int sk = sks[f];
+        if ((bits >> f) & 1u) {
+            j = __popc(bits & ((1u << f) - 1u));
+            if (sk == kNullSlot || nbs[f] < 0) sys.off[(size_t)j * C + c] = 0.0f;
+        }
         if (sk == kNullSlot) continue;
         const int k = sk >= 0 ? sk : ~sk;
         const int N = nbs[f];
@@ -273,7 +284,8 @@ __device__ __forceinline__ void pressure_assemble_body(const wcfd_mesh& m, const
             }
         }
     }
-    for (; j < m.ell_width; ++j) sys.off[(size_t)j * C + c] = 0.0f;
+    if (!bits)
+        for (; j < m.ell_width; ++j) sys.off[(size_t)j * C + c] = 0.0f;
     b += div[c];
     if (ref) {
         d = 1.0f;
@@ -303,21 +315,31 @@ void launch_pressure_assemble(bool xt, int grid, cudaStream_t st, const wcfd_mes
 }
 
 // y = A x on the mesh pattern; NC = 1 (scalar) or 3 (momentum: shared off-diagonals,
-// interleaved components).
+// interleaved components).  The first neighbour's product is rounded, the rest fused, in either
+// layout of the off-diagonals (row_product, common.cuh).
 template <int NC>
 __global__ void __launch_bounds__(kBlock) spmv_kernel(wcfd_mesh m, wcfd_system A, const float* __restrict__ x,
                                                       float* __restrict__ y) {
     const int c = blockIdx.x * kBlock + threadIdx.x;
     if (c >= m.n_cells) return;
     const int C = m.n_cells;
-    float acc[NC];
+    const bool in_place = slot_bits(m) != 0u;
+    float own[NC], acc[NC];
 #pragma unroll
-    for (int o = 0; o < NC; ++o) acc[o] = A.diag[NC * (size_t)c + o] * x[NC * (size_t)c + o];
+    for (int o = 0; o < NC; ++o) {
+        own[o] = x[NC * (size_t)c + o];
+        acc[o] = A.diag[NC * (size_t)c + o] * own[o];
+    }
+    bool begun = false;
     for (int j = 0; j < m.ell_width; ++j) {
         const float a = A.off[(size_t)j * C + c];
         const int col = __ldg(m.ell_col + (size_t)j * C + c);
 #pragma unroll
-        for (int o = 0; o < NC; ++o) acc[o] += a * x[NC * (size_t)col + o];
+        for (int o = 0; o < NC; ++o) {
+            const float xc = x[NC * (size_t)col + o];
+            acc[o] = begun ? fmaf(a, xc, acc[o]) : fmaf(A.diag[NC * (size_t)c + o], own[o], __fmul_rn(a, xc));
+        }
+        begun = begun || !in_place || a != 0.0f;
     }
 #pragma unroll
     for (int o = 0; o < NC; ++o) y[NC * (size_t)c + o] = acc[o];

@@ -13,6 +13,9 @@ using namespace wcfd;
 #ifndef WCFD_GRID_ROWS_PER_BLOCK
 #define WCFD_GRID_ROWS_PER_BLOCK 1024
 #endif
+#ifndef WCFD_CG_ROWS_PER_BLOCK
+#define WCFD_CG_ROWS_PER_BLOCK 512
+#endif
 
 namespace {
 
@@ -49,6 +52,8 @@ int check_mesh(const wcfd_mesh* m) {
         return set_error(WCFD_ERR_ARGUMENT, "faces_per_cell must be in 1..6");
     if (m->ell_width < 0 || m->ell_width > m->faces_per_cell)
         return set_error(WCFD_ERR_ARGUMENT, "ell_width must be in 0..faces_per_cell");
+    if (const unsigned bits = slot_bits(*m); bits >> m->faces_per_cell || (bits && __builtin_popcount(bits) != m->ell_width))
+        return set_error(WCFD_ERR_ARGUMENT, "slot_mask must name ell_width of the cells' slots");
     if (!m->face_owner || !m->face_nbr || !m->face_brow || !m->face_interp || !m->face_normal ||
         !m->face_gdiff || !m->face_rpf || !m->cell_slot || !m->cell_volume || !m->ell_col)
         return set_error(WCFD_ERR_ARGUMENT, "mesh has a null array");
@@ -65,25 +70,39 @@ GridCtl grid_ctl(double* partials) {
     return GridCtl{reinterpret_cast<unsigned*>(p), reinterpret_cast<int*>(p + 128), p + 256};
 }
 
-// co-resident blocks of a cooperative kernel on the current device (cached per kernel
-// and device)
-int coop_capacity(const void* fn, int /*unused*/) {
+// Co-resident blocks of a cooperative kernel on the current device, one per SM at most, and
+// the dynamic shared memory a block may take (its limit raised to that, for a kernel that
+// takes any); cached per kernel and device.
+struct CoopLimits {
+    int blocks;
+    size_t smem;
+};
+CoopLimits coop_limits(const void* fn, int threads, bool dynamic) {
     static std::mutex mu;
-    struct Entry { const void* fn; int dev; int cap; };
+    struct Entry { const void* fn; int dev; CoopLimits lim; };
     static Entry cache[64];
     static int n = 0;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
     for (int i = 0; i < n; ++i)
-        if (cache[i].fn == fn && cache[i].dev == dev) return cache[i].cap;
-    int per_sm = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSolverBlock, 0);
+        if (cache[i].fn == fn && cache[i].dev == dev) return cache[i].lim;
+    int per_sm = 0, sms = 0, optin = 0;
+    cudaFuncAttributes fa = {};
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncGetAttributes(&fa, fn);
+    CoopLimits lim = {0, dynamic && optin > (int)fa.sharedSizeBytes ? (size_t)optin - fa.sharedSizeBytes : 0};
+    if (lim.smem &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim.smem) != cudaSuccess) {
+        cudaGetLastError();
+        lim.smem = 0;
+    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, lim.smem);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int cap = per_sm * sms;
-    if (cap > kMaxGrid) cap = kMaxGrid;  // grid_reduce: one word per block and sum
-    if (n < 64) cache[n++] = Entry{fn, dev, cap};
-    return cap;
+    lim.blocks = per_sm > 0 ? sms : 0;
+    if (lim.blocks > kMaxGrid) lim.blocks = kMaxGrid;  // grid_reduce: one word per block and sum
+    if (n < 64) cache[n++] = Entry{fn, dev, lim};
+    return lim;
 }
 
 // Grid of a persistent kBlock-thread kernel over n items: every block resident at once
@@ -114,24 +133,31 @@ int resident_grid(const void* fn, long long n) {
     return want < cap ? (want < 1 ? 1 : want) : cap;
 }
 
-int launch_krylov(const void* fn, int slot, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws,
+int launch_krylov(bool cg, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws,
                   double atol, int maxiter, wcfd_solve_stats* stats, cudaStream_t st, const char* name,
                   double rtol = 0.0) {
     int rc = check_mesh(m);
     if (rc) return rc;
-    RET_IF(!fn, WCFD_ERR_ARGUMENT, "no solver kernel for this off-diagonal width");
     RET_IF(!A.diag || !A.off || !A.rhs || !x || !ws.vec || !ws.partials || !ws.barrier || !stats,
            WCFD_ERR_ARGUMENT, "null solver argument");
     // 16-byte words of the grid barrier
     RET_IF(reinterpret_cast<uintptr_t>(ws.partials) % 16 != 0, WCFD_ERR_ARGUMENT,
            "Krylov workspace: partials must be 16-byte aligned");
     RET_IF(maxiter < 0 || !(atol >= 0.0), WCFD_ERR_ARGUMENT, "bad atol or maxiter");
-    const int cap = coop_capacity(fn, slot);
+    // rows per block, then the kernel for them (a CG kernel's limits do not depend on it)
+    const int sms_cap = coop_limits(barrier_check_kernel_ptr(), kSolverBlock, false).blocks;
     LAUNCH_CHECK("occupancy query");
-    RET_IF(cap <= 0, WCFD_ERR_CUDA, "solver kernel cannot be resident");
-    long long want = (m->n_cells + WCFD_GRID_ROWS_PER_BLOCK - 1) / WCFD_GRID_ROWS_PER_BLOCK;
-    int grid = (int)(want < cap ? want : cap);
+    const int per_block = cg ? WCFD_CG_ROWS_PER_BLOCK : WCFD_GRID_ROWS_PER_BLOCK;
+    long long want = ((long long)m->n_cells + per_block - 1) / per_block;
+    int grid = (int)(want < sms_cap ? want : sms_cap);
     if (grid < 1) grid = 1;
+    const CgKernel ck = cg ? cg_kernel_for(m->ell_width, (int)(((long long)m->n_cells + grid - 1) / grid)) : CgKernel{nullptr, 0};
+    const void* fn = cg ? ck.fn : bicgstab_kernel_for(m->ell_width);
+    RET_IF(!fn, WCFD_ERR_ARGUMENT, "no solver kernel for this off-diagonal width");
+    const int threads = cg ? kCgBlock : kSolverBlock, chunk = ck.chunk;
+    const CoopLimits lim = coop_limits(fn, threads, cg);
+    LAUNCH_CHECK("occupancy query");
+    RET_IF(lim.blocks < grid, WCFD_ERR_CUDA, "solver kernel cannot be resident");
     if (cudaMemsetAsync(ws.partials, 0, kGridCtlBytes, st) != cudaSuccess)
         return set_error(WCFD_ERR_CUDA, "barrier reset failed");
     KrylovArgs a = {};
@@ -144,8 +170,29 @@ int launch_krylov(const void* fn, int slot, const wcfd_mesh* m, wcfd_system A, f
     a.rtol2 = rtol * rtol;
     a.maxiter = maxiter;
     a.stats = stats;
+    size_t smem = 0;
+    if (cg) {
+        // contiguous rows per block; shared memory goes to the column offsets first (16 or 32
+        // bytes per chunk), then to r, q and x (12 bytes a row for the 28 they move an
+        // iteration), then to 1/diag (4 for 4)
+        const long long rows = (((long long)m->n_cells + grid - 1) / grid + (chunk - 1)) / chunk * chunk;
+        a.rows = (int)rows;
+        grid = (int)((m->n_cells + rows - 1) / rows);
+        size_t left = lim.smem;
+        auto take = [&](size_t per_chunk, int most) {  // rows (a multiple of chunk)
+            const size_t fit = per_chunk ? left / per_chunk * chunk : (size_t)most;
+            const int n = fit < (size_t)most ? (int)fit : most;
+            left -= (size_t)(n / chunk) * per_chunk;
+            return n;
+        };
+        a.tab = take(cg_chunk_bytes(m->ell_width), a.rows);
+        a.part = take(3 * sizeof(float) * chunk, a.tab);
+        a.full = take(sizeof(float) * chunk, a.part);
+        smem = lim.smem - left;
+    }
     void* args[] = {&a};
-    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolverBlock), args, 0, st);
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s", name, cudaGetErrorString(e));
@@ -282,7 +329,7 @@ int wcfd_grid_barrier_check(int32_t skip_block, int32_t phases, int32_t* result,
     RET_IF(!result || phases < 1 || phases > 100000, WCFD_ERR_ARGUMENT, "bad phases or null result");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const void* fn = barrier_check_kernel_ptr();
-    const int cap = coop_capacity(fn, 0);
+    const int cap = coop_limits(fn, kSolverBlock, false).blocks;
     LAUNCH_CHECK("occupancy query");
     RET_IF(cap <= 0, WCFD_ERR_CUDA, "barrier check kernel cannot be resident");
     RET_IF(skip_block >= cap, WCFD_ERR_ARGUMENT, "skip_block beyond the grid");
@@ -556,7 +603,7 @@ static int cg_solve(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws 
     RET_IF(maxiter < 0 || !(atol >= 0.0) || !(rtol >= 0.0), WCFD_ERR_ARGUMENT, "bad tolerance or maxiter");
     rc = try_cluster_cg(m, A, x, atol, maxiter, stats, S(stream), rtol);
     if (rc >= 0) return rc;
-    return launch_krylov(cg_kernel_for(m->ell_width, m->ell_dcol != nullptr), 0, m, A, x, ws, atol, maxiter, stats, S(stream), "cg_kernel",
+    return launch_krylov(true, m, A, x, ws, atol, maxiter, stats, S(stream), "cg_kernel",
                          rtol);
 }
 
@@ -603,7 +650,7 @@ static int bicgstab_solve(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_kryl
                           int32_t maxiter, wcfd_solve_stats* stats, void* stream) {
     RET_IF(A.ncomp != 3, WCFD_ERR_ARGUMENT, "bicgstab solves the 3-component momentum system (ncomp 3)");
     RET_IF(!(rtol >= 0.0), WCFD_ERR_ARGUMENT, "bad rtol");
-    return launch_krylov(bicgstab_kernel_for(m->ell_width), 1, m, A, x, ws, atol, maxiter, stats, S(stream),
+    return launch_krylov(false, m, A, x, ws, atol, maxiter, stats, S(stream),
                          "bicgstab_kernel", rtol);
 }
 
@@ -773,5 +820,5 @@ extern "C" int wcfd_cg_noalloc(const wcfd_mesh* m, wcfd_system A, float* x, doub
     ws.partials = reinterpret_cast<double*>(b + kNoAllocPartialsOff);
     ws.results = nullptr;
     ws.barrier = reinterpret_cast<uint32_t*>(b + kNoAllocBarrierOff);
-    return launch_krylov(cg_kernel_for(m->ell_width, m->ell_dcol != nullptr), 0, m, A, x, ws, atol, maxiter, stats, S(stream), "cg_kernel");
+    return launch_krylov(true, m, A, x, ws, atol, maxiter, stats, S(stream), "cg_kernel");
 }

@@ -14,11 +14,17 @@ namespace wcfd {
 constexpr int kBlock = 256;      // threads of the one-thread-per-face/cell kernels
 constexpr int kMaxFieldBlock = 512;  // largest block of the batched field kernels (a launch parameter)
 constexpr int kSolverBlock = 1024;  // threads of the persistent Krylov kernels (one block per SM)
+constexpr int kCgBlock = 512;       // threads of the persistent CG (one block per SM)
 constexpr int kMaxSlots = 6;     // faces per cell (hex)
 // face reference of a null slot: a cell of a mixed mesh with fewer faces than the
 // mesh's faces_per_cell (a wedge or a tetrahedron among hexes); its weights are zero
 constexpr int kNullSlot = INT_MIN;
 constexpr int kClusterBlock = 1024;  // threads per CTA of the cluster-resident solver
+
+// the slot bits of a wcfd_mesh.slot_mask in use, else 0
+__host__ __device__ __forceinline__ unsigned slot_bits(const wcfd_mesh& m) {
+    return (m.slot_mask & 0xffff0000) == WCFD_SLOT_MASK ? (unsigned)m.slot_mask & 0xffffu : 0u;
+}
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -152,6 +158,30 @@ __device__ __forceinline__ float ff_div_to_float(const ff& an, const ff& bn) {
     const float rl = __fsub_rn(__fsub_rn(a.lo, e), __fmul_rn(q1, b.lo));
     const float q2 = __fdiv_rn(__fadd_rn(rh, rl), b.hi);
     return __fadd_rn(q1, q2);
+}
+
+// d p + sum_j o[j] g[j] of one matrix row, rounded as the compiler contracts the plain loop over
+// a row whose off-diagonals stand from slot 0 on: the first product is rounded, everything
+// after it is a fused multiply-add.  With the off-diagonals in place (in_place,
+// wcfd_mesh.slot_mask) a row beside a boundary may have its padding (coefficient 0) before its
+// first neighbour; that neighbour's product is then the rounded one, so that the layout does
+// not show in the result.
+template <int W>
+__device__ __forceinline__ float row_product(float d, float p, const float (&o)[W > 0 ? W : 1],
+                                             const float (&g)[W > 0 ? W : 1], bool in_place) {
+    if constexpr (W == 0) return __fmul_rn(d, p);
+    float q = fmaf(d, p, __fmul_rn(o[0], g[0]));
+#pragma unroll
+    for (int j = 1; j < W; ++j) q = fmaf(o[j], g[j], q);
+    if (in_place && o[0] == 0.0f) {
+        bool begun = false;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            q = begun ? fmaf(o[j], g[j], q) : fmaf(d, p, __fmul_rn(o[j], g[j]));
+            begun = begun || o[j] != 0.0f;
+        }
+    }
+    return q;
 }
 
 // Block total of NV float-float accumulators, still as float-float (the same bits in every

@@ -71,10 +71,18 @@ struct KrylovArgs {
     double rtol2;         // CG only: also stop when ||r||^2 <= rtol2 ||r0||^2 (0 = off)
     int maxiter;
     wcfd_solve_stats* stats;
+    // grid CG: rows per block and how many of a block's rows have their chunk's column offsets,
+    // r, q and x, and 1/diag in shared memory (multiples of the chunk, tab >= part >= full)
+    int rows, tab, part, full;
 };
 // kernel instantiations for off-diagonal width W (0..6), nullptr otherwise
-// delta: read the columns from wcfd_mesh.ell_dcol (int16 offsets from the row)
-const void* cg_kernel_for(int W, bool delta);
+// the grid CG for off-diagonal width W and about `rows` rows per block
+struct CgKernel {
+    const void* fn;
+    int chunk;  // rows a warp works on at a time
+};
+CgKernel cg_kernel_for(int W, int rows);
+size_t cg_chunk_bytes(int W);  // shared memory of a chunk's column offsets
 const void* barrier_check_kernel_ptr();
 const void* bicgstab_kernel_for(int W);
 const void* cg_cluster_kernel_for(int W, int R);

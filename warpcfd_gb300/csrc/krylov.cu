@@ -22,7 +22,8 @@
 
 namespace wcfd {
 
-constexpr int BS = kSolverBlock;
+constexpr int BS = kSolverBlock;  // threads of the BiCGSTAB
+constexpr int CGB = kCgBlock;     // threads of the CG
 
 __device__ __forceinline__ float jacobi(float d) { return d != 0.0f ? 1.0f / d : 1.0f; }
 
@@ -47,7 +48,7 @@ __device__ void fail_stats(const KrylovArgs& a, int k) {
 // (grid_reduce, common.cuh), thread 0 of which owns the scalars that follow from them
 #define REDUCE(NV, acc, ...)                                                  \
     do {                                                                      \
-        if (!grid_reduce<NV, BS>(a.g, acc, sbuf, ++phase, __VA_ARGS__)) {     \
+        if (!grid_reduce<NV, sizeof(sbuf) / sizeof(ff)>(a.g, acc, sbuf, ++phase, __VA_ARGS__)) { \
             fail_stats(a, sc.k);                                              \
             return;                                                           \
         }                                                                     \
@@ -100,76 +101,162 @@ __device__ __forceinline__ void prefetch_matrix_lines(const int* col, const floa
     }
 }
 
-// Column of slot j of row i: from the int16 offsets (kD, wcfd_mesh.ell_dcol) or the int32
-// columns, streamed (evict-first) or with a plain load.
-template <bool kD, bool kStream>
-__device__ __forceinline__ int ell_column(const int* __restrict__ col, const int16_t* __restrict__ dcol, size_t idx,
-                                          int i) {
-    if constexpr (kD) return i + (int)(kStream ? __ldcs(dcol + idx) : dcol[idx]);
-    else return kStream ? __ldcs(col + idx) : col[idx];
+// Columns of row i, slot by slot: from the int16 offsets (wcfd_mesh.ell_dcol) when the mesh has
+// them (half the bytes), else the int32 columns.  Every load is issued before the first use.
+template <int W>
+__device__ __forceinline__ void ell_columns(int (&c)[W > 0 ? W : 1], const int* __restrict__ col,
+                                            const int16_t* __restrict__ dcol, int C, int i) {
+    if (dcol) {
+#pragma unroll
+        for (int j = 0; j < W; ++j) c[j] = __ldcs(dcol + (size_t)j * C + i);
+#pragma unroll
+        for (int j = 0; j < W; ++j) c[j] += i;
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) c[j] = __ldcs(col + (size_t)j * C + i);
+    }
 }
 
+// Rows of the grid CG are worked on in chunks of kChunk consecutive rows by one warp, lane `lane`
+// taking the rows lane, lane + 32, ... of it.  A chunk is regular when in each off-diagonal
+// slot all its rows have the same column offset (or no neighbour: zero coefficient, own
+// column) and every row of it exists: with the off-diagonals in place (wcfd_mesh.slot_mask)
+// a structured numbering's chunks are, beside boundaries too.  The offsets are written down
+// once per solve; a regular chunk then needs no column loads and one address per slot for
+// all of a lane's rows.  An irregular chunk reads its columns from the mesh.
+template <int W>
+struct alignas(16) ChunkCols {
+    int d[W > 4 ? 8 : 4];  // d[0] = kIrregular: not regular
+};
+constexpr int kIrregular = INT_MIN;
+
 // Jacobi-preconditioned CG on a scalar system, W = off-diagonal width known at compile
-// time so the loads of a row's columns and gathered values are all in flight at once.
-// Workspace: r, pA, pB, q, invd, z (6 C floats).
+// time so the loads of a row's coefficients and gathered values are all in flight at once.
+// Workspace: r, pA, pB, q, invd, z (6 C floats; r, q and invd only of rows that do not fit
+// shared memory).
 //
-// The matrix (off-diagonals and columns, 8 W bytes a row) is read with the streaming
-// (evict-first) cache policy: it is re-read every iteration but does not fit L2 next to
-// the vectors on large meshes, and evicting it first keeps the vectors (gathered and
-// re-read within the iteration) resident in the 129 MB L2.
+// Block b owns the rows [b R, (b + 1) R) for the whole solve, warp w of it the chunks w,
+// w + CGB / 32, ... of those.  What only the owner of a row touches stays in shared memory,
+// for as many of the block's rows as fit (KrylovArgs::part rows: r, q, x; full rows: 1/diag
+// too): a 128^3 system's x, r and q lie in the 152 SMs' shared memory whole.
 //
 // Per iteration: (1) p_new = z + beta p_old for the row and every neighbour, q = A p_new,
 // p.q -- and x += alpha_prev p_old, the previous iteration's solution update, which reads
-// the p_old this pass loads anyway; (2) r -= alpha q, z = r / diag, r.r and r.z.  Each
-// thread takes two rows (i, i + stride) per trip of pass (1) so that twice the column,
-// coefficient and gather loads are in flight: the pass is bound by memory latency, not
-// by bandwidth, at one row per thread.
+// the p_old this pass loads anyway; (2) r -= alpha q, z = r / diag, r.r and r.z.
 //
-// kD: the columns come from the int16 offsets (wcfd_mesh.ell_dcol) instead of the int32
-// columns, 6 W instead of 8 W streamed bytes per row (the same columns, the same bits):
-// pass (1) streams the matrix from DRAM while the vectors stay in L2, so on the 128^3
-// cavity (W = 6) an iteration went from 35.5 to 33.3 us.  The BiCGSTAB keeps the int32
-// columns: the offsets made its solve slower there (0.338 -> 0.360 ms).
-template <int W, bool kD>
-__global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
+// NR, the rows of a lane in a chunk: a block's rows are best covered in one pass over them (the
+// loads of all are then in flight at once), so NR follows the rows per block up to 4
+// (cg_kernel_for).  Measured per iteration: 1,000 rows per block (61x47x53 hexes) 5.2 us with
+// NR = 2, 5.8 with 3; 1,064 (30x31x29x6 tetrahedra) 6.0 with 3, 6.7 with 2; 1,628 (cylinder)
+// 6.2 with 4, 7.0 with 2; on more rows than 4 per thread 3 is the fastest (128^3: 22.4 us,
+// 23.2 with 2, 26.0 with 1,024 threads of one row each).
+template <int W, int NR>
+__global__ void __launch_bounds__(CGB, 1) cg_kernel(KrylovArgs a) {
+    extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ KScalars sc;
-    __shared__ ff sbuf[2 * BS / 2];
+    __shared__ ff sbuf[2 * CGB / 2];
+    constexpr int WA = W > 0 ? W : 1;  // no zero-length arrays for W = 0
+    constexpr int kChunk = 32 * NR;    // rows of a warp at a time
+    constexpr int STEP = CGB / 32 * kChunk;
     const int C = a.m.n_cells;
-    float* r = a.ws;
-    float* pbuf[2] = {a.ws + (size_t)C, a.ws + 2 * (size_t)C};
-    float* q = a.ws + 3 * (size_t)C;
-    float* invd = a.ws + 4 * (size_t)C;
-    float* z = a.ws + 5 * (size_t)C;
+    const int t = threadIdx.x, lane = t & 31;
+    const int row0 = blockIdx.x * a.rows;
+    const int nloc = min(a.rows, C - row0);
+    const int part = a.part, full = a.full, tab = W > 0 ? a.tab : 0;
+    ChunkCols<W>* cols = reinterpret_cast<ChunkCols<W>*>(dyn);
+    float* s_r = reinterpret_cast<float*>(cols + tab / kChunk);
+    float* s_q = s_r + part;
+    float* s_x = s_q + part;
+    float* s_i = s_x + part;
+    float* const r = a.ws;
+    float* const pA = a.ws + (size_t)C;
+    float* const pB = a.ws + 2 * (size_t)C;
+    float* const q = a.ws + 3 * (size_t)C;
+    float* const invd = a.ws + 4 * (size_t)C;
+    float* const z = a.ws + 5 * (size_t)C;
     const float* __restrict__ b = a.A.rhs;
     const float* __restrict__ diag = a.A.diag;
     const float* __restrict__ off = a.A.off;
     const int* __restrict__ col = a.m.ell_col;
     const int16_t* __restrict__ dcol = a.m.ell_dcol;
     float* x = a.x;
-    const int stride = gridDim.x * BS;
-    const int i0 = blockIdx.x * BS + threadIdx.x;
+    const int lw = (t >> 5) * kChunk;  // this warp's first chunk
+    const bool in_place = slot_bits(a.m) != 0u;
     unsigned phase = 0;
-    if (threadIdx.x == 0) {
+    if (t == 0) {
         sc.k = 0;
         sc.status = WCFD_OK;
     }
 
-    // r = b - A x ; z = M r ; p = z ; rr = r.r ; rz = r.z ; bb = b.b
+    // r = b - A x ; z = M r ; p = z ; rr = r.r ; rz = r.z ; bb = b.b ; the chunks' offsets
     ff acc[2] = {ff_zero(), ff_zero()}, accb[1] = {ff_zero()};
-    for (int i = i0; i < C; i += stride) {
-        float ax = diag[i] * x[i];
+    for (int l0 = lw; l0 < nloc; l0 += STEP) {
+        int d[WA];
+        unsigned seen = 0;
+        bool regular = l0 + kChunk <= nloc;
 #pragma unroll
-        for (int j = 0; j < W; ++j) ax += off[(size_t)j * C + i] * x[ell_column<kD, false>(col, dcol, (size_t)j * C + i, i)];
-        const float ri = b[i] - ax;
-        const float di = jacobi(diag[i]);
-        const float zi = ri * di;
-        r[i] = ri;
-        invd[i] = di;
-        z[i] = zi;
-        pbuf[0][i] = zi;
-        ff_fma(acc[0], ri, ri);
-        ff_fma(acc[1], ri, zi);
-        ff_fma(accb[0], b[i], b[i]);
+        for (int j = 0; j < W; ++j) d[j] = 0;
+        int c[NR][WA];
+        float o[NR][WA], xc[NR][WA];
+#pragma unroll
+        for (int k = 0; k < NR; ++k) {
+            const int i = row0 + min(l0 + 32 * k + lane, nloc - 1);
+            ell_columns<W>(c[k], col, dcol, C, i);
+#pragma unroll
+            for (int j = 0; j < W; ++j) o[k][j] = off[(size_t)j * C + i];
+        }
+#pragma unroll
+        for (int k = 0; k < NR; ++k)
+#pragma unroll
+            for (int j = 0; j < W; ++j) xc[k][j] = x[c[k][j]];
+#pragma unroll
+        for (int k = 0; k < NR; ++k) {
+            const int l = l0 + 32 * k + lane;
+            const int i = row0 + min(l, nloc - 1);
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                // the slot's offset: the first one seen in the chunk
+                const bool real = c[k][j] != i;
+                const unsigned has = __ballot_sync(0xffffffffu, real);
+                if (!((seen >> j) & 1u) && has) {
+                    d[j] = __shfl_sync(0xffffffffu, c[k][j] - i, __ffs(has) - 1);
+                    seen |= 1u << j;
+                }
+                // (a caller's matrix may hold a coefficient on the own column of a padding slot)
+                regular = regular && (real ? c[k][j] - i == d[j] : o[k][j] == 0.0f);
+            }
+            if (l >= nloc) continue;
+            const float xi = x[i], di = diag[i];
+            const float ax = row_product<W>(di, xi, o[k], xc[k], in_place);
+            const float bi = b[i];
+            const float ri = bi - ax;
+            const float vi = jacobi(di);
+            const float zi = ri * vi;
+            if (l0 < part) {
+                s_r[l] = ri;
+                s_x[l] = xi;
+            } else {
+                r[i] = ri;
+            }
+            if (l0 < full) s_i[l] = vi;
+            else invd[i] = vi;
+            z[i] = zi;
+            pA[i] = zi;
+            ff_fma(acc[0], ri, ri);
+            ff_fma(acc[1], ri, zi);
+            ff_fma(accb[0], bi, bi);
+        }
+        if (l0 < tab) {
+            // the rows' addresses all lie in the vectors, absent neighbours' included
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+                regular = regular && row0 + l0 + (long long)d[j] >= 0 && row0 + l0 + kChunk - 1 + (long long)d[j] < C;
+            regular = __all_sync(0xffffffffu, regular);
+            if (lane == 0) {
+#pragma unroll
+                for (int j = 0; j < W; ++j) cols[l0 / kChunk].d[j] = regular ? d[j] : kIrregular;
+            }
+        }
     }
     REDUCE(1, accb, [&](const ff* s) {
         if (threadIdx.x == 0 && blockIdx.x == 0) a.stats->rhs_norm = sqrt(ff_to_double(s[0]));
@@ -185,52 +272,67 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
     while (sc.go) {
         const float bf = sc.bf;
         const float ap = pending;
-        const float* po = pbuf[cur];  // written by other blocks in this launch: no restrict
-        float* pn = pbuf[cur ^ 1];
+        const float* po = cur ? pB : pA;  // written by other blocks in this launch: no restrict
+        float* pn = cur ? pA : pB;
         // x += alpha_prev p_old ; p_new = z + beta p_old (row and neighbours) ; q = A p_new ; p.q
         ff accq[1] = {ff_zero()};
-        for (int i = i0; i < C; i += 2 * stride) {
-            const int i2 = i + stride;
-            const bool two = i2 < C;
-            const int k2 = two ? i2 : i;  // a lone last row loads itself twice, stores once
-            constexpr int WA = W > 0 ? W : 1;  // no zero-length arrays for W = 0
-            int c1[WA], c2[WA];
-            float o1[WA], o2[WA];
+        for (int l0 = lw; l0 < nloc; l0 += STEP) {
+            const int l = l0 + lane, i = row0 + l;
+            const bool inside = l0 + kChunk <= nloc;
+            float o[NR][WA], zc[NR][WA], pc[NR][WA], zo[NR], poi[NR], dd[NR];
 #pragma unroll
-            for (int j = 0; j < W; ++j) {
-                c1[j] = ell_column<kD, true>(col, dcol, (size_t)j * C + i, i);
-                c2[j] = ell_column<kD, true>(col, dcol, (size_t)j * C + k2, k2);
+            for (int k = 0; k < NR; ++k) {
+                const int ik = row0 + min(l + 32 * k, nloc - 1);
+#pragma unroll
+                for (int j = 0; j < W; ++j) o[k][j] = __ldg(off + (size_t)j * C + ik);
+                dd[k] = diag[ik];
+            }
+            if (W > 0 && l0 < tab && cols[l0 / kChunk].d[0] != kIrregular) {
+                const ChunkCols<W> rec = cols[l0 / kChunk];
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    const float* zj = z + i + rec.d[j];
+                    const float* pj = po + i + rec.d[j];
+#pragma unroll
+                    for (int k = 0; k < NR; ++k) {
+                        zc[k][j] = zj[32 * k];
+                        pc[k][j] = pj[32 * k];
+                    }
+                }
+            } else {
+                int c[NR][WA];
+#pragma unroll
+                for (int k = 0; k < NR; ++k) ell_columns<W>(c[k], col, dcol, C, row0 + min(l + 32 * k, nloc - 1));
+#pragma unroll
+                for (int k = 0; k < NR; ++k)
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        zc[k][j] = z[c[k][j]];
+                        pc[k][j] = po[c[k][j]];
+                    }
             }
 #pragma unroll
-            for (int j = 0; j < W; ++j) {
-                o1[j] = __ldcs(off + (size_t)j * C + i);
-                o2[j] = __ldcs(off + (size_t)j * C + k2);
-            }
-            const float po1 = po[i], po2 = po[k2];
-            const float p1 = z[i] + bf * po1;
-            const float p2 = z[k2] + bf * po2;
-            float q1 = diag[i] * p1;
-            float q2 = diag[k2] * p2;
-            float g1[WA], g2[WA];
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                g1[j] = z[c1[j]] + bf * po[c1[j]];
-                g2[j] = z[c2[j]] + bf * po[c2[j]];
+            for (int k = 0; k < NR; ++k) {
+                if (!inside && l + 32 * k >= nloc) continue;
+                zo[k] = z[i + 32 * k];
+                poi[k] = po[i + 32 * k];
             }
 #pragma unroll
-            for (int j = 0; j < W; ++j) {
-                q1 += o1[j] * g1[j];
-                q2 += o2[j] * g2[j];
-            }
-            if (ap != 0.0f) x[i] += ap * po1;
-            pn[i] = p1;
-            q[i] = q1;
-            ff_fma(accq[0], p1, q1);
-            if (two) {
-                if (ap != 0.0f) x[i2] += ap * po2;
-                pn[i2] = p2;
-                q[i2] = q2;
-                ff_fma(accq[0], p2, q2);
+            for (int k = 0; k < NR; ++k) {
+                if (!inside && l + 32 * k >= nloc) continue;
+                const float pi = zo[k] + bf * poi[k];
+#pragma unroll
+                for (int j = 0; j < W; ++j) zc[k][j] += bf * pc[k][j];
+                const float qi = row_product<W>(dd[k], pi, o[k], zc[k], in_place);
+                if (l0 < part) {
+                    if (ap != 0.0f) s_x[l + 32 * k] += ap * poi[k];
+                    s_q[l + 32 * k] = qi;
+                } else {
+                    if (ap != 0.0f) x[i + 32 * k] += ap * poi[k];
+                    q[i + 32 * k] = qi;
+                }
+                pn[i + 32 * k] = pi;
+                ff_fma(accq[0], pi, qi);
             }
         }
         REDUCE(1, accq, [&](const ff* pq) {
@@ -247,13 +349,25 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
         const float af = sc.af;
         // r -= alpha q ; z = M r ; rr ; rz
         ff acc2[2] = {ff_zero(), ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-            const float ri = r[i] - af * q[i];
-            r[i] = ri;
-            const float zi = ri * invd[i];
-            z[i] = zi;
-            ff_fma(acc2[0], ri, ri);
-            ff_fma(acc2[1], ri, zi);
+        for (int l0 = lw; l0 < nloc; l0 += STEP) {
+            const int l = l0 + lane, i = row0 + l;
+            const bool inside = l0 + kChunk <= nloc;
+#pragma unroll
+            for (int k = 0; k < NR; ++k) {
+                if (!inside && l + 32 * k >= nloc) continue;
+                float ri;
+                if (l0 < part) {
+                    ri = s_r[l + 32 * k] - af * s_q[l + 32 * k];
+                    s_r[l + 32 * k] = ri;
+                } else {
+                    ri = r[i + 32 * k] - af * q[i + 32 * k];
+                    r[i + 32 * k] = ri;
+                }
+                const float zi = ri * (l0 < full ? s_i[l + 32 * k] : invd[i + 32 * k]);
+                z[i + 32 * k] = zi;
+                ff_fma(acc2[0], ri, ri);
+                ff_fma(acc2[1], ri, zi);
+            }
         }
         REDUCE(2, acc2, [&](const ff* s) {
             if (threadIdx.x != 0) return;
@@ -266,10 +380,14 @@ __global__ void __launch_bounds__(BS, 1) cg_kernel(KrylovArgs a) {
         pending = af;
         cur ^= 1;
     }
-    // the last iteration's x += alpha p (its p is pbuf[cur] after the swap)
-    if (pending != 0.0f) {
-        const float* pl = pbuf[cur];
-        for (int i = i0; i < C; i += stride) x[i] += pending * pl[i];
+    // the last iteration's x += alpha p (its p is the current buffer's)
+    const float* pl = cur ? pB : pA;
+    for (int l0 = lw; l0 < nloc; l0 += STEP) {
+        for (int l = l0 + lane; l < min(l0 + kChunk, nloc); l += 32) {
+            const int i = row0 + l;
+            if (l0 < part) x[i] = pending != 0.0f ? s_x[l] + pending * pl[i] : s_x[l];
+            else if (pending != 0.0f) x[i] += pending * pl[i];
+        }
     }
     write_stats(a, sc);
 }
@@ -295,6 +413,8 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
     const float* __restrict__ off = a.A.off;
     const int* __restrict__ col = a.m.ell_col;
     float* x = a.x;
+    constexpr int WA = W > 0 ? W : 1;
+    const bool in_place = slot_bits(a.m) != 0u;
     const int stride = gridDim.x * BS;
     const int i0 = blockIdx.x * BS + threadIdx.x;
     unsigned phase = 0;
@@ -306,16 +426,17 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
     // r = b - A x ; r0 = r ; p = r ; v = 0 ; rr ; rho = r0.r = rr ; bb = b.b
     ff acc[2] = {ff_zero(), ff_zero()};
     for (int i = i0; i < C; i += stride) {
-        float ax[3];
-#pragma unroll
-        for (int o = 0; o < 3; ++o) ax[o] = diag[3 * (size_t)i + o] * x[3 * (size_t)i + o];
+        float ax[3], v[WA], g[3][WA];
 #pragma unroll
         for (int j = 0; j < W; ++j) {
-            const float v = __ldcs(off + (size_t)j * C + i);
+            v[j] = __ldcs(off + (size_t)j * C + i);
             const int c = __ldcs(col + (size_t)j * C + i);
 #pragma unroll
-            for (int o = 0; o < 3; ++o) ax[o] += v * x[3 * (size_t)c + o];
+            for (int o = 0; o < 3; ++o) g[o][j] = x[3 * (size_t)c + o];
         }
+#pragma unroll
+        for (int o = 0; o < 3; ++o)
+            ax[o] = row_product<W>(diag[3 * (size_t)i + o], x[3 * (size_t)i + o], v, g[o], in_place);
 #pragma unroll
         for (int o = 0; o < 3; ++o) {
             const size_t q = 3 * (size_t)i + o;
@@ -348,23 +469,27 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
         ff accv[1] = {ff_zero()};
         for (int i = i0; i < C; i += stride) {
             prefetch_matrix_lines<W>(col, off, C, stride, i, 1);
-            float pi[3], vi[3];
+            float pi[3], vi[3], v[WA], g[3][WA];
 #pragma unroll
             for (int o = 0; o < 3; ++o) {
                 const size_t q = 3 * (size_t)i + o;
                 pi[o] = r[q] + bf * (po[q] - of0 * vo[q]);
-                vi[o] = diag[q] * (pi[o] * invd[q]);
             }
 #pragma unroll
             for (int j = 0; j < W; ++j) {
-                const float v = __ldcs(off + (size_t)j * C + i);
+                v[j] = __ldcs(off + (size_t)j * C + i);
                 const int c = __ldcs(col + (size_t)j * C + i);
 #pragma unroll
                 for (int o = 0; o < 3; ++o) {
                     const size_t q = 3 * (size_t)c + o;
                     const float pc = r[q] + bf * (po[q] - of0 * vo[q]);
-                    vi[o] += v * (pc * invd[q]);
+                    g[o][j] = pc * invd[q];
                 }
+            }
+#pragma unroll
+            for (int o = 0; o < 3; ++o) {
+                const size_t q = 3 * (size_t)i + o;
+                vi[o] = row_product<W>(diag[q], pi[o] * invd[q], v, g[o], in_place);
             }
 #pragma unroll
             for (int o = 0; o < 3; ++o) {
@@ -390,24 +515,24 @@ __global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
         ff acct[2] = {ff_zero(), ff_zero()};
         for (int i = i0; i < C; i += stride) {
             prefetch_matrix_lines<W>(col, off, C, stride, i, 1);
-            float si[3], ti[3];
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                si[o] = r[q] - af * vn[q];
-                x[q] += af * (pn[q] * invd[q]);
-                ti[o] = diag[q] * (si[o] * invd[q]);
-            }
+            float si[3], ti[3], v[WA], g[3][WA];
 #pragma unroll
             for (int j = 0; j < W; ++j) {
-                const float v = __ldcs(off + (size_t)j * C + i);
+                v[j] = __ldcs(off + (size_t)j * C + i);
                 const int c = __ldcs(col + (size_t)j * C + i);
 #pragma unroll
                 for (int o = 0; o < 3; ++o) {
                     const size_t q = 3 * (size_t)c + o;
                     const float scv = r[q] - af * vn[q];
-                    ti[o] += v * (scv * invd[q]);
+                    g[o][j] = scv * invd[q];
                 }
+            }
+#pragma unroll
+            for (int o = 0; o < 3; ++o) {
+                const size_t q = 3 * (size_t)i + o;
+                si[o] = r[q] - af * vn[q];
+                ti[o] = row_product<W>(diag[q], si[o] * invd[q], v, g[o], in_place);
+                x[q] += af * (pn[q] * invd[q]);
             }
 #pragma unroll
             for (int o = 0; o < 3; ++o) {
@@ -538,17 +663,16 @@ __global__ void __launch_bounds__(BS, 1) barrier_check_kernel(GridCtl g, int ski
 
 const void* barrier_check_kernel_ptr() { return (const void*)barrier_check_kernel; }
 
-// W = 0 has no columns to read: its offset form is the plain one
-template <bool kD>
+template <int NR>
 const void* cg_kernel_pick(int W) {
     switch (W) {
-        case 0: return (const void*)cg_kernel<0, false>;
-        case 1: return (const void*)cg_kernel<1, kD>;
-        case 2: return (const void*)cg_kernel<2, kD>;
-        case 3: return (const void*)cg_kernel<3, kD>;
-        case 4: return (const void*)cg_kernel<4, kD>;
-        case 5: return (const void*)cg_kernel<5, kD>;
-        case 6: return (const void*)cg_kernel<6, kD>;
+        case 0: return (const void*)cg_kernel<0, NR>;
+        case 1: return (const void*)cg_kernel<1, NR>;
+        case 2: return (const void*)cg_kernel<2, NR>;
+        case 3: return (const void*)cg_kernel<3, NR>;
+        case 4: return (const void*)cg_kernel<4, NR>;
+        case 5: return (const void*)cg_kernel<5, NR>;
+        case 6: return (const void*)cg_kernel<6, NR>;
         default: return nullptr;
     }
 }
@@ -566,6 +690,16 @@ const void* bicgstab_kernel_for(int W) {
     }
 }
 
-const void* cg_kernel_for(int W, bool delta) { return delta ? cg_kernel_pick<true>(W) : cg_kernel_pick<false>(W); }
+size_t cg_chunk_bytes(int W) { return W > 4 ? sizeof(ChunkCols<5>) : W > 0 ? sizeof(ChunkCols<4>) : 0; }
+
+CgKernel cg_kernel_for(int W, int rows) {
+    switch ((rows + CGB - 1) / CGB) {
+        case 0:
+        case 1: return CgKernel{cg_kernel_pick<1>(W), 32};
+        case 2: return CgKernel{cg_kernel_pick<2>(W), 64};
+        case 4: return CgKernel{cg_kernel_pick<4>(W), 128};
+        default: return CgKernel{cg_kernel_pick<3>(W), 96};
+    }
+}
 
 }  // namespace wcfd

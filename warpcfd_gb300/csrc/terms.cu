@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(kBlock) assemble_terms_kernel(wcfd_mesh m, wcf
     const int c = blockIdx.x * kBlock + threadIdx.x;
     const int C = m.n_cells, F = m.faces_per_cell, W = m.ell_width, n = sys.ncomp;
     if (c >= C) return;
+    const unsigned bits = slot_bits(m);
     float dg[3] = {0.0f, 0.0f, 0.0f}, b[3] = {0.0f, 0.0f, 0.0f};
     float od[kMaxSlots];
 #pragma unroll
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(kBlock) assemble_terms_kernel(wcfd_mesh m, wcf
         for (int f = 0; f < F; ++f) {
             const SlotFace sf = slot_face(m, c, f);
             if (sf.null_) continue;
+            if (bits) j = __popc(bits & ((1u << f) - 1u));
             const float* e = w + ((size_t)c * F + f) * n * 3;
             for (int o = 0; o < n; ++o) dg[o] += sc * e[3 * o];
             if (__ldg(m.face_nbr + sf.k) >= 0) {
