@@ -141,3 +141,29 @@ def test_rows_past_shared_memory_and_coefficients_on_padding():
     x, st = _solve(col, off, diag, rhs, 0b111111, maxiter=500, atol=1e-3)
     r = _residual(col, off, diag, rhs, x)
     assert st["status"] == 0 and abs(r - st["residual"]) <= 500 * 6e-8 * 14.0 * float(x.double().norm())
+
+
+# one CTA to sixteen, 1 to 8 rows of a thread and ragged last CTAs, around the cluster CG's
+# 512, 1,024 and 2,048 rows per CTA
+@pytest.mark.parametrize("n", [(7, 1, 1), (64, 8, 1), (129, 4, 1), (91, 90, 1), (100, 164, 1), (181, 181, 1), (205, 160, 1),
+                               (26, 25, 24), (32, 32, 32), (33, 32, 32)])
+def test_cluster_solve_matches_the_grid_solve(n):
+    """Both solve to ||r|| <= 1e-3; diagonal dominance >= 0.01 bounds each error by 1e-3 / 0.01.
+    The reported residual norms are those of the solutions up to the recurrence's rounding (see
+    above)."""
+    from warpcfd_gb300 import _lib
+    cc, oc = _compact(*_box(n)[:2])
+    _, _, diag, rhs = _box(n)
+    a, sa = _solve(cc, oc, diag, rhs, maxiter=500, atol=1e-3)
+    _lib.call("wcfd_set_krylov_path", 2)
+    try:
+        b, sb = _solve(cc, oc, diag, rhs, maxiter=500, atol=1e-3)
+        c, sc = _solve(cc, oc, diag, rhs, maxiter=500, atol=1e-3)
+    finally:
+        _lib.call("wcfd_set_krylov_path", 1)
+    assert sa["status"] == 0 and sb["status"] == 0
+    assert torch.equal(b, c) and sb == sc
+    assert float((a.double() - b.double()).norm()) <= 2 * 1e-3 / 0.01
+    bound = 500 * 6e-8 * 14.0 * float(b.double().norm())
+    assert abs(_residual(cc, oc, diag, rhs, b) - sb["residual"]) <= bound
+    assert abs(sb["rhs_norm"] - float(rhs.double().norm())) <= 1e-6 * sb["rhs_norm"]

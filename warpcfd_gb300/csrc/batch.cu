@@ -67,12 +67,12 @@ int prepare_cluster(const void* fn, size_t smem) {
     return WCFD_OK;
 }
 
-int launch_cluster(const void* fn, int n_cases, int cs, size_t smem, cudaStream_t st, void** args) {
+int launch_cluster(const void* fn, int n_cases, int cs, int threads, size_t smem, cudaStream_t st, void** args) {
     const int rc = prepare_cluster(fn, smem);
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_cases * cs);
-    cfg.blockDim = dim3(kClusterBlock);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -121,8 +121,11 @@ __global__ void __launch_bounds__(kMaxFieldBlock) refine_update_batched(const wc
 const void* batch_cg_kernel(const wcfd_batch_dims& d, int R) {
     return d.cg_variant == 1 ? cg1m_cluster_batched_for(d.ell_width, R) : cg_cluster_batched_for(d.ell_width, R);
 }
+int batch_cg_threads(const wcfd_batch_dims& d, int R) {
+    return d.cg_variant == 1 ? kClusterBlock : cluster_cg_threads(R, true);
+}
 size_t batch_cg_smem(const wcfd_batch_dims& d, int R) {
-    return d.cg_variant == 1 ? cluster_cg1m_smem_bytes(R, d.ell_width) : cluster_cg_smem_bytes(R, d.ell_width);
+    return d.cg_variant == 1 ? cluster_cg1m_smem_bytes(R, d.ell_width) : cluster_cg_smem_bytes(R, d.ell_width, true);
 }
 
 #define BCHECK(what)                                                                               \
@@ -206,7 +209,7 @@ extern "C" int wcfd_batch_simple_iteration(const wcfd_case* cases, int32_t n_cas
     BCHECK("momentum_assemble_batched");
     int csv = cs;
     void* bargs[] = {(void*)&cases, &csv};
-    int rc = launch_cluster(bi_fn, n_cases, cs, 0, st, bargs);
+    int rc = launch_cluster(bi_fn, n_cases, cs, kClusterBlock, 0, st, bargs);
     if (rc) return rc;
     // :118-123
     hbya_batched<<<gc, fb, 0, st>>>(cases);
@@ -228,7 +231,7 @@ extern "C" int wcfd_batch_simple_iteration(const wcfd_case* cases, int32_t n_cas
                     refine_residual_batched<<<gc, fb, 0, st>>>(cases);
                     BCHECK("refine_residual_batched");
                     void* cargs[] = {(void*)&cases, &csv, &one};
-                    rc = launch_cluster(cg_fn, n_cases, cs, smem, st, cargs);
+                    rc = launch_cluster(cg_fn, n_cases, cs, batch_cg_threads(d, R), smem, st, cargs);
                     if (rc) return rc;
                     refine_update_batched<<<gc, fb, 0, st>>>(cases);
                     BCHECK("refine_update_batched");
@@ -236,7 +239,7 @@ extern "C" int wcfd_batch_simple_iteration(const wcfd_case* cases, int32_t n_cas
             } else {
                 int zero = 0;
                 void* cargs[] = {(void*)&cases, &csv, &zero};
-                rc = launch_cluster(cg_fn, n_cases, cs, smem, st, cargs);
+                rc = launch_cluster(cg_fn, n_cases, cs, batch_cg_threads(d, R), smem, st, cargs);
                 if (rc) return rc;
             }
             p_update_batched<<<gc, fb, 0, st>>>(cases);

@@ -116,4 +116,71 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
     }
 }
 
+// The same sums for CTAs of 256 threads, to every thread (normalised, the same bits): every
+// thread stores its value, warp 0 merges eight each (l, l+32, ..., pairwise), then by butterfly,
+// and stores the CTA total into a slot of every CTA (DSMEM); after the cluster barrier every
+// warp merges the cs <= 16 slots, so that no block barrier and no broadcast follows: the eight
+// warps form the scalars redundantly.  With the caller's four accumulators per thread merged
+// as cluster_reduce_tree merges its quarters (narrow_merge), the sums are those of that tree
+// bit for bit.  (Every warp storing its own total to every CTA, eight times the remote stores:
+// 2,000-2,400 cycles a reduction on 16 CTAs against 1,900.)
+// sbuf: [kClusterSums][256]; slots: [2][kClusterSums][16], double-buffered by `parity`; remote:
+// the address of slots in CTA `lane` (any CTA for lanes past the cluster).
+constexpr int kClusterSums = 3;
+constexpr int kNarrowBlock = 256;
+template <int NV>
+__device__ __forceinline__ void cluster_reduce_narrow(ff (&v)[NV], ff* sbuf, const ff* slots, uint32_t remote,
+                                                      unsigned parity, unsigned me, unsigned cs) {
+    static_assert(NV <= kClusterSums && kNarrowBlock == 256, "eight warps");
+    const int t = threadIdx.x, lane = t & 31;
+    const unsigned base = parity * (kClusterSums * 16);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) sbuf[i * kNarrowBlock + t] = v[i];
+    __syncthreads();
+    if (t < 32) {
+        ff y[NV][8];
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) y[i][k] = sbuf[i * kNarrowBlock + 32 * k + t];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) ff_tree(y[i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) ff_shfl_merge(y[i][0], o);
+        if ((unsigned)t < cs)
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                st_cluster_v2f32(remote + (base + i * 16 + me) * (unsigned)sizeof(ff), y[i][0].hi, y[i][0].lo);
+    }
+    cluster_sync_warp0_release();
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = (unsigned)(lane & 15) < cs ? slots[base + i * 16 + (lane & 15)] : ff_zero();
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) ff_shfl_merge(v[i], o);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = ff_norm(v[i]);
+}
+// a thread's accumulators of the rows t + 256 (4 m + q), q = 0..3, in acc[q]
+__device__ __forceinline__ ff narrow_merge(ff (&acc)[4]) {
+    ff_merge(acc[0], acc[1]);
+    ff_merge(acc[2], acc[3]);
+    ff_merge(acc[0], acc[2]);
+    return acc[0];
+}
+
+__device__ __forceinline__ float2 ld_shared_f32x2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float2 ld_cluster_f32x2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+    return v;
+}
+
 }  // namespace wcfd

@@ -88,7 +88,8 @@ const void* bicgstab_kernel_for(int W);
 const void* cg_cluster_kernel_for(int W, int R);
 const void* cg_cluster_batched_for(int W, int R);
 const void* bicgstab_cluster_batched_for(int W);
-size_t cluster_cg_smem_bytes(int R, int W);
+size_t cluster_cg_smem_bytes(int R, int W, bool batched);
+int cluster_cg_threads(int R, bool batched);
 int cluster_cg_max_rows(int W, int optin);
 int cluster_cg_rpt(int R);
 const void* cg1_cluster_kernel_for(int W, int R);

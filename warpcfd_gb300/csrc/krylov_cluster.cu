@@ -1,23 +1,29 @@
 // Cluster-resident CG: one thread-block cluster (up to 16 CTAs) holds the whole scalar
-// system in shared memory for the length of the solve.
+// system on chip for the length of the solve.
 //
-//  * CTA q of the cluster owns rows [q R, (q+1) R); its slice of the matrix (off-diagonals,
-//    packed (rank, local) columns, diagonal) and the gathered vectors (z and p, stored as
-//    (z, p) pairs so one 8-byte load fetches both) live in its shared memory; x, r and q of
-//    a thread's own rows stay in registers.
+//  * CTA q of the cluster owns rows [q R, (q+1) R).  Up to 2,048 rows a CTA, eight warps keep
+//    their rows' off-diagonals, neighbour addresses, x, r, q and p in registers, up to eight
+//    rows a thread (cg_cluster_body); beyond that, and in the batched form, 1,024 threads keep
+//    the matrix in shared memory (cg_cluster_wide_body; a case's sums must not depend on the
+//    largest case beside it, so the batched form has one thread count).  What others gather,
+//    z and p of every row, is in shared memory, as (z, p) pairs that one 8-byte load fetches.
 //  * A neighbour value owned by another CTA is read through distributed shared memory
 //    (mapa + ld.shared::cluster); nothing touches global memory between the set-up and
 //    the final write of x.
 //  * Grid-wide synchronisation is the hardware cluster barrier
-//    (barrier.cluster.arrive.release / wait.acquire).  A dot product is reduced by a
-//    shared-memory tree in each CTA (exact products in float-float, common.cuh); warp 0
-//    stores the CTA total into a slot of every CTA's shared memory and after the barrier
-//    merges the cs slots in a fixed order, so all CTAs (and all runs) agree bit for bit.
-//    Thread 0 forms alpha and beta from the float-float sums and broadcasts them.  All
-//    CTAs take the same branch at every test, so no CTA can leave while another still
-//    waits or reads its memory.
+//    (barrier.cluster.arrive.release / wait.acquire), inside the reductions (cluster.cuh): exact
+//    products in float-float (common.cuh), merged in a fixed order, so all CTAs (and all runs)
+//    agree bit for bit.  All CTAs take the same branch at every test, so no CTA can leave
+//    while another still waits or reads its memory.
 //  * The direction update p = z + beta p is evaluated inside the SpMV for the row and its
-//    neighbours (double-buffered p), so an iteration needs two barriers.
+//    neighbours, so an iteration needs two barriers.
+// Bound by the latency of its two reductions and, with many rows a CTA, by shared-memory
+// bandwidth.  Measured per iteration (1,024 threads with everything in shared memory ->
+// eight warps with the matrix in registers): 2 CTAs x 512 rows 2.72 -> 1.65 us, 8 x 512 2.88 ->
+// 1.78, 16 x 2,000 3.77 -> 3.1.  Eight warps are few enough to merge the CTAs' sums and form the
+// scalars redundantly, without a hop through one thread; with 32 warps the same takes 4,600
+// cycles a reduction instead of 2,300, hence the two reductions.  4,096 rows a CTA with the
+// matrix in registers (512 threads x 8 rows) spill: 7.8 us against 4.7.
 // The arithmetic is that of cg_kernel (krylov.cu): the same Jacobi-preconditioned CG with
 // fp64-accurate dot products and the same stop test.
 #include "cluster.cuh"
@@ -26,12 +32,16 @@
 
 namespace wcfd {
 
-// Dynamic shared memory per CTA for R rows and width W: the reduction tree (3 x 1024
-// float-float values), then per row the pairs (z, p) of two iteration buffers (16), the
-// off-diagonals (4 W), diag and 1/diag (8) and 16-bit packed columns (2 W).  x, r and q
-// live in registers (each thread owns the same rows for the whole solve).  16 CTAs of
-// R <= 4096 rows hold 65536 rows of width 4.
-size_t cluster_cg_smem_bytes(int R, int W) {
+// rows per CTA that eight warps hold in registers, eight to a thread
+constexpr int kNarrowRows = 8 * kNarrowBlock;
+int cluster_cg_threads(int R, bool batched) { return batched || R > kNarrowRows ? CBS : kNarrowBlock; }
+
+// Dynamic shared memory per CTA for R rows and width W: the (z, p) pairs (8 bytes a row), or, for
+// the wide form, the reduction tree (3 x 1024 float-float values), then per row the pairs of
+// two iteration buffers (16), the off-diagonals (4 W), diag and 1/diag (8) and 16-bit packed
+// columns (2 W).  16 CTAs of R <= 4096 rows hold 65536 rows of width 4.
+size_t cluster_cg_smem_bytes(int R, int W, bool batched) {
+    if (!batched && R <= kNarrowRows) return (size_t)R * 8;
     return 3 * (size_t)CBS * sizeof(ff) + (size_t)R * (6 * (size_t)W + 24);
 }
 
@@ -47,14 +57,181 @@ int cluster_cg_max_rows(int W, int optin) {
 // rows per thread for R rows per CTA
 int cluster_cg_rpt(int R) { return R <= CBS ? 1 : (R <= 2 * CBS ? 2 : 4); }
 
-__device__ __forceinline__ float2 ld_cluster_f32x2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-    return v;
+template <int W, int RPT>
+__device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ ff slots[2 * kClusterSums * 16], sbuf[kClusterSums * kNarrowBlock];
+    constexpr int T = kNarrowBlock;
+    constexpr int WA = W > 0 ? W : 1;
+    constexpr int GR = RPT < 4 ? RPT : 4;
+    const int C = a.m.n_cells;
+    const unsigned me = cluster_rank();
+    const unsigned cs = cluster_nranks();
+    const int row0 = (int)me * R;
+    const int nloc = max(0, min(R, C - row0));
+    float2* zp = reinterpret_cast<float2*>(smem);              // [R] (z, p)
+    const int t = threadIdx.x;
+    const uint32_t remote = map_rank(slots, min((unsigned)(t & 31), cs - 1));
+    const uint32_t zp0 = (uint32_t)__cvta_generic_to_shared(zp);
+
+    // the matrix rows of this thread; where a neighbour's pair lies: its address, own or another
+    // CTA's
+    float o[RPT][WA], dg[RPT], iv[RPT];
+    uint32_t at[RPT][WA];
+#pragma unroll
+    for (int u = 0; u < RPT; ++u)  // a row past the end gathers the CTA's first pair, unused
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            at[u][j] = zp0;
+        }
+    unsigned local = 0;  // bit u: no row of this warp's u-th 32 has a neighbour in another CTA
+    float xr[RPT], rr_[RPT], qr[RPT], pr[RPT];
+    // r = b - A x (x read from global) ; z = M r ; the first direction is z (p_old = 0) ; rr ; rz ; bb
+    ff arr[4], arz[4], abb[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) arr[q] = arz[q] = abb[q] = ff_zero();
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+        const int l = t + u * T;
+        rr_[u] = qr[u] = pr[u] = 0.0f;
+        xr[u] = 0.0f;
+        bool mine = true;
+        if (l < nloc) {
+            const int g = row0 + l;
+            const float d = a.A.diag[g];
+            const float di = d != 0.0f ? 1.0f / d : 1.0f;
+            float ov[WA], xc[WA];
+            dg[u] = d;
+            iv[u] = di;
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                ov[j] = a.A.off[(size_t)j * C + g];
+                o[u][j] = ov[j];
+                const int c = a.m.ell_col[(size_t)j * C + g];
+                const int rk = c / R, lo = c - rk * R;
+                xc[j] = a.x[c];
+                mine = mine && rk == (int)me;
+                at[u][j] = rk == (int)me ? zp0 + 8u * lo : map_rank(zp + lo, rk);
+            }
+            const float xi = a.x[g], bi = a.A.rhs[g];
+            xr[u] = xi;
+            const float ri = bi - row_product<W>(d, xi, ov, xc, false);
+            const float zi = ri * di;
+            rr_[u] = ri;
+            zp[l] = make_float2(zi, 0.0f);
+            ff_fma(arr[u % 4], ri, ri);
+            ff_fma(arz[u % 4], ri, zi);
+            ff_fma(abb[u % 4], bi, bi);
+        }
+        if (__all_sync(0xffffffffu, mine)) local |= 1u << u;
+    }
+    unsigned parity = 0;
+    ff acc[3] = {narrow_merge(arr), narrow_merge(arz), narrow_merge(abb)};
+    cluster_reduce_narrow<3>(acc, sbuf, slots, remote, parity, me, cs);
+    parity ^= 1u;
+    ff rr = acc[0], rz = acc[1];
+    const ff thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * ff_to_double(rr))));
+    if (me == 0 && t == 0) {
+        a.stats->initial_residual = sqrt(ff_to_double(rr));
+        a.stats->rhs_norm = sqrt(ff_to_double(acc[2]));
+    }
+    float bf = 0.0f;
+    int k = 0, status = WCFD_OK;
+    while (k < a.maxiter && ff_gt(rr, thr2)) {
+        // p = z + beta p_old (own row and each neighbour) ; q = A p ; p.q.  The gathers of GR rows
+        // are issued before the first is used.
+        ff apq[4] = {ff_zero(), ff_zero(), ff_zero(), ff_zero()};
+#pragma unroll
+        for (int u0 = 0; u0 < RPT; u0 += GR) {
+            float2 v[GR][WA];
+#pragma unroll
+            for (int q = 0; q < GR; ++q) {
+                const int u = u0 + q;
+                uint32_t ad[WA];
+                if ((local >> u) & 1u) {  // warp-uniform: every neighbour in this CTA
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        ad[j] = at[u][j];
+                        v[q][j] = ld_shared_f32x2(ad[j]);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        ad[j] = at[u][j];
+                        v[q][j] = ld_cluster_f32x2(ad[j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < GR; ++q) {
+                const int u = u0 + q, l = t + u * T;
+                if (l >= nloc) continue;
+                float d, zi;  // z as it was formed
+                d = dg[u];
+                zi = __fmul_rn(rr_[u], iv[u]);
+                const float pi = fmaf(bf, pr[u], zi);
+                float qi = __fmul_rn(d, pi);
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    float oj;
+                    oj = o[u][j];
+                    qi = fmaf(oj, fmaf(bf, v[q][j].y, v[q][j].x), qi);
+                }
+                pr[u] = pi;
+                qr[u] = qi;
+                ff_fma(apq[u % 4], pi, qi);
+            }
+        }
+        ff accq[1] = {narrow_merge(apq)};
+        cluster_reduce_narrow<1>(accq, sbuf, slots, remote, parity, me, cs);
+        parity ^= 1u;
+        if (accq[0].hi == 0.0f) {
+            status = WCFD_KRYLOV_BREAKDOWN;
+            break;
+        }
+        const float af = ff_div_to_float(rz, accq[0]);
+        // x += alpha p ; r -= alpha q ; z = M r ; rr ; rz
+#pragma unroll
+        for (int q = 0; q < 4; ++q) arr[q] = arz[q] = ff_zero();
+#pragma unroll
+        for (int u = 0; u < RPT; ++u) {
+            const int l = t + u * T;
+            if (l < nloc) {
+                xr[u] = fmaf(af, pr[u], xr[u]);
+                const float ri = fmaf(-af, qr[u], rr_[u]);
+                float zi;
+                zi = __fmul_rn(ri, iv[u]);
+                rr_[u] = ri;
+                zp[l] = make_float2(zi, pr[u]);
+                ff_fma(arr[u % 4], ri, ri);
+                ff_fma(arz[u % 4], ri, zi);
+            }
+        }
+        ff acc2[2] = {narrow_merge(arr), narrow_merge(arz)};
+        cluster_reduce_narrow<2>(acc2, sbuf, slots, remote, parity, me, cs);
+        parity ^= 1u;
+        rr = acc2[0];
+        bf = rz.hi != 0.0f ? ff_div_to_float(acc2[1], rz) : 0.0f;
+        rz = acc2[1];
+        ++k;
+    }
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+        const int l = t + u * T;
+        if (l < nloc) {
+            a.x[row0 + l] = xr[u];
+        }
+    }
+    if (me == 0 && t == 0) {
+        if (status == WCFD_OK && !ff_le(rr, thr2)) status = WCFD_NOT_CONVERGED;
+        a.stats->iterations = k;
+        a.stats->status = status;
+        a.stats->residual = sqrt(ff_to_double(rr));
+    }
 }
 
 template <int W, int RPT>
-__device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
+__device__ __forceinline__ void cg_cluster_wide_body(const KrylovArgs& a, int R) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ff slots[2 * 3 * 16];
     __shared__ unsigned char chunk_local[4096 / 32];  // 32-row chunk with no off-CTA neighbour
@@ -240,8 +417,13 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
 }
 
 template <int W, int RPT>
-__global__ void __launch_bounds__(CBS) cg_cluster_kernel(KrylovArgs a, int R) {
+__global__ void __launch_bounds__(kNarrowBlock, 1) cg_cluster_kernel(KrylovArgs a, int R) {
     cg_cluster_body<W, RPT>(a, R);
+}
+
+template <int W, int RPT>
+__global__ void __launch_bounds__(CBS) cg_cluster_wide_kernel(KrylovArgs a, int R) {
+    cg_cluster_wide_body<W, RPT>(a, R);
 }
 
 // One cluster per case of a device case table: the pressure CG of every case
@@ -265,7 +447,7 @@ __global__ void __launch_bounds__(CBS) cg_cluster_batched(const wcfd_case* __res
     }
     a.maxiter = c.prm.maxiter;
     a.stats = c.stats + 1;
-    cg_cluster_body<W, RPT>(a, (c.mesh.n_cells + cs - 1) / cs);
+    cg_cluster_wide_body<W, RPT>(a, (c.mesh.n_cells + cs - 1) / cs);
 }
 
 // BiCGSTAB on one case per cluster, for the batched form: the momentum system of the
@@ -501,34 +683,35 @@ __global__ void __launch_bounds__(CBS) bicgstab_cluster_batched(const wcfd_case*
         default: return nullptr;                 \
     }
 
-#define WCFD_WR_SWITCH(NAME)                                   \
-    switch (W * 8 + cluster_cg_rpt(R)) {                       \
-        case 0 * 8 + 1: return (const void*)NAME<0, 1>;        \
-        case 0 * 8 + 2: return (const void*)NAME<0, 2>;        \
-        case 0 * 8 + 4: return (const void*)NAME<0, 4>;        \
-        case 1 * 8 + 1: return (const void*)NAME<1, 1>;        \
-        case 1 * 8 + 2: return (const void*)NAME<1, 2>;        \
-        case 1 * 8 + 4: return (const void*)NAME<1, 4>;        \
-        case 2 * 8 + 1: return (const void*)NAME<2, 1>;        \
-        case 2 * 8 + 2: return (const void*)NAME<2, 2>;        \
-        case 2 * 8 + 4: return (const void*)NAME<2, 4>;        \
-        case 3 * 8 + 1: return (const void*)NAME<3, 1>;        \
-        case 3 * 8 + 2: return (const void*)NAME<3, 2>;        \
-        case 3 * 8 + 4: return (const void*)NAME<3, 4>;        \
-        case 4 * 8 + 1: return (const void*)NAME<4, 1>;        \
-        case 4 * 8 + 2: return (const void*)NAME<4, 2>;        \
-        case 4 * 8 + 4: return (const void*)NAME<4, 4>;        \
-        case 5 * 8 + 1: return (const void*)NAME<5, 1>;        \
-        case 5 * 8 + 2: return (const void*)NAME<5, 2>;        \
-        case 5 * 8 + 4: return (const void*)NAME<5, 4>;        \
-        case 6 * 8 + 1: return (const void*)NAME<6, 1>;        \
-        case 6 * 8 + 2: return (const void*)NAME<6, 2>;        \
-        case 6 * 8 + 4: return (const void*)NAME<6, 4>;        \
-        default: return nullptr;                               \
+// the kernel for R rows a CTA: the fewest rows per thread that cover them
+template <int W>
+const void* pick_kernel(int R, bool batched) {
+    if (batched) {
+        if (R <= CBS) return (const void*)cg_cluster_batched<W, 1>;
+        if (R <= 2 * CBS) return (const void*)cg_cluster_batched<W, 2>;
+        return (const void*)cg_cluster_batched<W, 4>;
     }
+    if (R <= 512) return (const void*)cg_cluster_kernel<W, 2>;
+    if (R <= 1024) return (const void*)cg_cluster_kernel<W, 4>;
+    if (R <= kNarrowRows) return (const void*)cg_cluster_kernel<W, 8>;
+    return (const void*)cg_cluster_wide_kernel<W, 4>;
+}
 
-const void* cg_cluster_batched_for(int W, int R) { WCFD_WR_SWITCH(cg_cluster_batched) }
+static const void* cg_cluster_pick(int W, int R, bool batched) {
+    if (R > 4096) return nullptr;  // 12-bit local index of the packed columns
+    switch (W) {
+        case 0: return pick_kernel<0>(R, batched);
+        case 1: return pick_kernel<1>(R, batched);
+        case 2: return pick_kernel<2>(R, batched);
+        case 3: return pick_kernel<3>(R, batched);
+        case 4: return pick_kernel<4>(R, batched);
+        case 5: return pick_kernel<5>(R, batched);
+        case 6: return pick_kernel<6>(R, batched);
+        default: return nullptr;
+    }
+}
+const void* cg_cluster_kernel_for(int W, int R) { return cg_cluster_pick(W, R, false); }
+const void* cg_cluster_batched_for(int W, int R) { return cg_cluster_pick(W, R, true); }
 const void* bicgstab_cluster_batched_for(int W) { WCFD_W_SWITCH(bicgstab_cluster_batched) }
-const void* cg_cluster_kernel_for(int W, int R) { WCFD_WR_SWITCH(cg_cluster_kernel) }
 
 }  // namespace wcfd
