@@ -19,8 +19,8 @@
 //    neighbours, so an iteration needs two barriers.
 // Bound by the latency of its two reductions and, with many rows a CTA, by shared-memory
 // bandwidth.  Measured per iteration (1,024 threads with everything in shared memory ->
-// eight warps with the matrix in registers): 2 CTAs x 512 rows 2.72 -> 1.65 us, 8 x 512 2.88 ->
-// 1.78, 16 x 2,000 3.77 -> 3.1.  Eight warps are few enough to merge the CTAs' sums and form the
+// eight warps with the matrix in registers): 2 CTAs x 512 rows 2.76 -> 1.57 us, 8 x 512 2.88 ->
+// 1.64, 16 x 2,000 3.77 -> 2.7.  Eight warps are few enough to merge the CTAs' sums and form the
 // scalars redundantly, without a hop through one thread; with 32 warps the same takes 4,600
 // cycles a reduction instead of 2,300, hence the two reductions.  4,096 rows a CTA with the
 // matrix in registers (512 threads x 8 rows) spill: 7.8 us against 4.7.
@@ -36,12 +36,13 @@ namespace wcfd {
 constexpr int kNarrowRows = 8 * kNarrowBlock;
 int cluster_cg_threads(int R, bool batched) { return batched || R > kNarrowRows ? CBS : kNarrowBlock; }
 
-// Dynamic shared memory per CTA for R rows and width W: the (z, p) pairs (8 bytes a row), or, for
+// Dynamic shared memory per CTA for R rows and width W: the (z, p) pairs (8 bytes a row,
+// of all the rows its threads can hold), or, for
 // the wide form, the reduction tree (3 x 1024 float-float values), then per row the pairs of
 // two iteration buffers (16), the off-diagonals (4 W), diag and 1/diag (8) and 16-bit packed
 // columns (2 W).  16 CTAs of R <= 4096 rows hold 65536 rows of width 4.
 size_t cluster_cg_smem_bytes(int R, int W, bool batched) {
-    if (!batched && R <= kNarrowRows) return (size_t)R * 8;
+    if (!batched && R <= kNarrowRows) return 8 * (size_t)(R <= 512 ? 512 : R <= 1024 ? 1024 : 2048);
     return 3 * (size_t)CBS * sizeof(ff) + (size_t)R * (6 * (size_t)W + 24);
 }
 
@@ -69,8 +70,9 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
     const unsigned cs = cluster_nranks();
     const int row0 = (int)me * R;
     const int nloc = max(0, min(R, C - row0));
-    float2* zp = reinterpret_cast<float2*>(smem);              // [R] (z, p)
+    float2* zp = reinterpret_cast<float2*>(smem);  // [RPT T] (z, p)
     const int t = threadIdx.x;
+    const int groups = (nloc + GR * T - 1) / (GR * T);  // groups of GR rows a thread that hold any
     const uint32_t remote = map_rank(slots, min((unsigned)(t & 31), cs - 1));
     const uint32_t zp0 = (uint32_t)__cvta_generic_to_shared(zp);
 
@@ -78,12 +80,6 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
     // CTA's
     float o[RPT][WA], dg[RPT], iv[RPT];
     uint32_t at[RPT][WA];
-#pragma unroll
-    for (int u = 0; u < RPT; ++u)  // a row past the end gathers the CTA's first pair, unused
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            at[u][j] = zp0;
-        }
     unsigned local = 0;  // bit u: no row of this warp's u-th 32 has a neighbour in another CTA
     float xr[RPT], rr_[RPT], qr[RPT], pr[RPT];
     // r = b - A x (x read from global) ; z = M r ; the first direction is z (p_old = 0) ; rr ; rz ; bb
@@ -93,8 +89,15 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
         const int l = t + u * T;
-        rr_[u] = qr[u] = pr[u] = 0.0f;
-        xr[u] = 0.0f;
+        // a row past the end is a row of zeros that gathers its own pair (0, 0): the passes need
+        // no test of the row, which would keep a thread's rows from overlapping
+        xr[u] = rr_[u] = qr[u] = pr[u] = dg[u] = iv[u] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            o[u][j] = 0.0f;
+            at[u][j] = zp0 + 8u * l;
+        }
+        float zi = 0.0f;
         bool mine = true;
         if (l < nloc) {
             const int g = row0 + l;
@@ -116,13 +119,13 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             const float xi = a.x[g], bi = a.A.rhs[g];
             xr[u] = xi;
             const float ri = bi - row_product<W>(d, xi, ov, xc, false);
-            const float zi = ri * di;
+            zi = ri * di;
             rr_[u] = ri;
-            zp[l] = make_float2(zi, 0.0f);
             ff_fma(arr[u % 4], ri, ri);
             ff_fma(arz[u % 4], ri, zi);
             ff_fma(abb[u % 4], bi, bi);
         }
+        zp[l] = make_float2(zi, 0.0f);
         if (__all_sync(0xffffffffu, mine)) local |= 1u << u;
     }
     unsigned parity = 0;
@@ -143,6 +146,7 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
         ff apq[4] = {ff_zero(), ff_zero(), ff_zero(), ff_zero()};
 #pragma unroll
         for (int u0 = 0; u0 < RPT; u0 += GR) {
+            if (u0 >= groups * GR) break;
             float2 v[GR][WA];
 #pragma unroll
             for (int q = 0; q < GR; ++q) {
@@ -164,13 +168,10 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
 #pragma unroll
             for (int q = 0; q < GR; ++q) {
-                const int u = u0 + q, l = t + u * T;
-                if (l >= nloc) continue;
-                float d, zi;  // z as it was formed
-                d = dg[u];
-                zi = __fmul_rn(rr_[u], iv[u]);
+                const int u = u0 + q;
+                const float zi = __fmul_rn(rr_[u], iv[u]);  // as it was formed
                 const float pi = fmaf(bf, pr[u], zi);
-                float qi = __fmul_rn(d, pi);
+                float qi = __fmul_rn(dg[u], pi);
 #pragma unroll
                 for (int j = 0; j < W; ++j) {
                     float oj;
@@ -194,15 +195,15 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) arr[q] = arz[q] = ff_zero();
 #pragma unroll
-        for (int u = 0; u < RPT; ++u) {
-            const int l = t + u * T;
-            if (l < nloc) {
+        for (int u0 = 0; u0 < RPT; u0 += GR) {
+            if (u0 >= groups * GR) break;
+#pragma unroll
+            for (int u = u0; u < u0 + GR; ++u) {
                 xr[u] = fmaf(af, pr[u], xr[u]);
                 const float ri = fmaf(-af, qr[u], rr_[u]);
-                float zi;
-                zi = __fmul_rn(ri, iv[u]);
+                const float zi = __fmul_rn(ri, iv[u]);
                 rr_[u] = ri;
-                zp[l] = make_float2(zi, pr[u]);
+                zp[t + u * T] = make_float2(zi, pr[u]);
                 ff_fma(arr[u % 4], ri, ri);
                 ff_fma(arz[u % 4], ri, zi);
             }

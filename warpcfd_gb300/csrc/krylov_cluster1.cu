@@ -233,92 +233,189 @@ const void* cg1_cluster_kernel_for(int W, int R) {
 }
 
 // ---------------------------------------------------------------------------------
-// The single-reduction CG for the batched form, up to 4,096 rows per CTA (RPT <= 4).
+// The single-reduction CG for the batched form, up to 4,096 rows per CTA.
 //
 // The (r, w, s, 1/d) double buffer above takes 32 bytes of shared memory per row, too many
-// for the 4,096 rows per CTA of the batched form's largest cases.  Here only u = M r lives
-// in shared memory (a single buffer), and an iteration is two phases:
+// for the 4,096 rows per CTA of the batched form's largest cases.  Here only u = M r is
+// gathered (a single buffer in shared memory), and an iteration is two phases:
 //   (1) s = w + beta s ; p = u + beta p ; x += alpha p ; r -= alpha s ; u = M r, for the own
-//       rows (registers, and u into shared memory), then a cluster barrier (release /
-//       acquire) so that every CTA's new u is visible;
+//       rows (registers, and u into shared memory), then a barrier (of the cluster; of the block
+//       when the cluster is one CTA) so that every CTA's new u is visible;
 //   (2) w = A u (the neighbours' u from shared memory, DSMEM for another CTA's rows) and
 //       r.r, r.u, w.u, in ONE cluster all-reduce.
 // The barrier inside the all-reduce also keeps phase (1) of the next iteration from
-// overwriting a u that another CTA still gathers.  Per iteration that is one plain cluster
-// barrier and one all-reduce instead of the two all-reduces of textbook CG.  The values are
-// those of cg1_cluster_body (the same operations per row); the scalar recurrences and the
-// stop test are its own.
-// Shared memory: the reduction tree, then per row u (4), off-diagonals (4 W), diag and 1/diag
-// (8) and the 16-bit packed columns (2 W).
+// overwriting a u that another CTA still gathers.  The values are those of cg1_cluster_body
+// (the same operations per row); the scalar recurrences and the stop test are its own.
+//
+// Few warps with many rows each: 256 threads of up to 8 rows, with the whole matrix in
+// registers, or 512 of 8 (the addresses of the gathered u in registers, off-diagonals and
+// diagonals in shared memory, one 16-byte load a row at width 4).  Cycles of an iteration at
+// 4,096 rows on one CTA, 1,024 threads with everything in shared memory -> this form: update
+// 1,259 -> 788, barrier 1,116 -> 109, SpMV and products 4,082 -> 3,031, reduction 2,865 -> 1,027,
+// scalars 894 -> 940.  Bound by instruction issue (about 120 a row and iteration, half of them
+// the exact products); groups of rows that a smaller case of the batch does not have are
+// skipped whole.
+template <int RPT, int T>
+constexpr bool kMatrixInRegisters = RPT * T <= 2048;
+
+static int cg1m_capacity(int R) { return R <= 512 ? 512 : R <= 1024 ? 1024 : R <= 2048 ? 2048 : 4096; }
+int cluster_cg1m_threads(int R) { return R <= 2048 ? 256 : 512; }
+// dynamic shared memory: u (4 bytes a row); past 2,048 rows the off-diagonals, diag and 1/diag
+// too, laid out by thread
 size_t cluster_cg1m_smem_bytes(int R, int W) {
-    return 3 * (size_t)CBS * sizeof(ff) + (size_t)R * (6 * (size_t)W + 12);
+    const int cap = cg1m_capacity(R);
+    return 4 * (size_t)cap + (cap > 2048 ? (4 * (size_t)W + 8) * cap : 0);
 }
 
-template <int W, int RPT>
+// Row of thread t's u-th in a CTA of T threads, and the accumulator it adds to: chosen so that
+// merging a thread's accumulators and then the threads' (cg1m_reduce) is the tree of
+// cluster_reduce_tree over 1,024 threads that own the rows t, t + 1024, ... -- the same sums bit
+// for bit whatever T and RPT are, so a case's result does not depend on the kernel that its
+// batch's largest case asks for.
+template <int T>
+__device__ __forceinline__ int cg1m_row(int t, int u) {
+    if constexpr (T == 256) return t + 256 * u;
+    else return (t & 255) + ((t >> 8) << 9) + 256 * (u & 1) + 1024 * (u >> 1);
+}
+template <int T>
+constexpr int kCg1mAcc = T == 256 ? 4 : 2;
+
+// Sum three float-float values over the cluster's CTAs, the sums (normalised, the same bits) to
+// thread 0.  acc[i][q]: the accumulators of value i.  Warp i merges value i over the CTA's
+// threads and stores it to every CTA's slots; a cluster of one CTA needs neither DSMEM nor
+// the cluster barrier.  sbuf: [3][T]; slots: [2][3][16], double-buffered by `parity`.
+template <int T>
+__device__ __forceinline__ void cg1m_reduce(ff (&acc)[3][kCg1mAcc<T>], ff (&out)[3], ff* sbuf, ff* slots, unsigned parity,
+                                            unsigned me, unsigned cs) {
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const unsigned base = parity * 48;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        ff_merge(acc[i][0], acc[i][1]);
+        if constexpr (T == 256) {
+            ff_merge(acc[i][2], acc[i][3]);
+            ff_merge(acc[i][0], acc[i][2]);
+        }
+        sbuf[i * T + t] = acc[i][0];
+    }
+    __syncthreads();
+    if (wid < 3) {
+        ff y[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) y[k] = sbuf[wid * T + 32 * k + lane];
+        if constexpr (T == 512) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) ff_merge(y[k], sbuf[wid * T + 256 + 32 * k + lane]);
+        }
+        ff_tree(y);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(y[0], o);
+        if ((unsigned)lane < cs) st_cluster_v2f32(map_rank(slots + base + wid * 16 + me, lane), y[0].hi, y[0].lo);
+    }
+    if (cs > 1) cluster_sync_all();
+    else __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) out[i] = (unsigned)lane < cs ? slots[base + i * 16 + lane] : ff_zero();
+        if (cs > 1) {
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)  // lanes 0..15 hold the cs <= 16 slots
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ff_shfl_merge(out[i], o);
+        }
+    }
+}
+
+template <int W, int RPT, int T>
 __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ ff slots[2 * 3 * 16];
-    __shared__ unsigned char chunk_local[4096 / 32];  // 32-row chunk with no off-CTA neighbour
+    __shared__ ff slots[2 * 3 * 16], sbuf[3 * T];
     struct Scal {
         ff rr, gamma, thr2;
         float af, bf, alpha_prev;
         int go, status, k;
     };
     __shared__ Scal sc;
+    constexpr int WA = W > 0 ? W : 1, NA = kCg1mAcc<T>, GR = RPT < 1024 / T ? RPT : 1024 / T;
+    constexpr bool REG = kMatrixInRegisters<RPT, T>;
+    constexpr int RM = REG ? RPT : 1;
     const int C = a.m.n_cells;
     const unsigned me = cluster_rank();
     const unsigned cs = cluster_nranks();
     const int row0 = (int)me * R;
     const int nloc = max(0, min(R, C - row0));
-    ff* sbuf = reinterpret_cast<ff*>(smem);                 // [3][CBS]
-    float* ub = reinterpret_cast<float*>(sbuf + 3 * CBS);   // [R] u = M r
-    float* off = ub + R;                                    // [W][R]
-    float* diag = off + W * R;
-    float* invd = diag + R;
-    uint16_t* colp = reinterpret_cast<uint16_t*>(invd + R);  // [W][R] (rank << 12) | local
+    float* ub = reinterpret_cast<float*>(smem);   // [RPT T] u = M r, by row
+    float* s_o = ub + RPT * T;                    // [RPT][T][W] (W = 4) or [RPT][W][T], by thread (!REG)
+    float* s_d = s_o + W * RPT * T;               // [RPT][T]
+    float* s_i = s_d + RPT * T;                   // [RPT][T]
     const int t0 = threadIdx.x;
+    const int groups = (nloc + GR * T - 1) / (GR * T);  // groups of GR rows a thread that hold any
+    const uint32_t ub0 = (uint32_t)__cvta_generic_to_shared(ub);
 
-    for (int l = t0; l < nloc; l += CBS) {
-        const int g = row0 + l;
-        const float d = a.A.diag[g];
-        diag[l] = d;
-        invd[l] = d != 0.0f ? 1.0f / d : 1.0f;
-        bool local = true;
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            off[j * R + l] = a.A.off[(size_t)j * C + g];
-            const int c = a.m.ell_col[(size_t)j * C + g];
-            const int rk = c / R;
-            colp[j * R + l] = (uint16_t)((rk << 12) | (c - rk * R));
-            local = local && rk == (int)me;
-        }
-        local = __all_sync(__activemask(), local);
-        if ((t0 & 31) == 0) chunk_local[l >> 5] = local ? 1 : 0;
-    }
+    // this thread's rows of the matrix; at: where a neighbour's u lies, here or in another CTA
+    float o[RM][WA], dg[RM], iv[RM];
+    uint32_t at[RPT][WA];
+    unsigned local = 0;  // bit u: no row of this warp's u-th 32 has a neighbour in another CTA
+    float xr[RPT], pr[RPT], sr[RPT], rr_[RPT], wr[RPT], ur[RPT];
     // r0 = b - A x0 ; u0 = M r0 ; r0.r0 ; b.b
-    float xr[RPT], pr[RPT], sr[RPT], rr_[RPT], wr[RPT];
-    ff acc[3] = {ff_zero(), ff_zero(), ff_zero()};
+    ff acc[3][NA];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int q = 0; q < NA; ++q) acc[i][q] = ff_zero();
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
-        const int l = t0 + u * CBS;
-        xr[u] = pr[u] = sr[u] = rr_[u] = wr[u] = 0.0f;
+        const int l = cg1m_row<T>(t0, u);
+        xr[u] = pr[u] = sr[u] = rr_[u] = wr[u] = ur[u] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < W; ++j) at[u][j] = ub0 + 4u * l;
+        bool mine = true;
+        // a row past the end is a row of zeros that gathers its own u = 0: the passes need no
+        // test of the row, which would keep a lane's rows from overlapping
+        float d = 0.0f, di = 0.0f, ov[WA];
+#pragma unroll
+        for (int j = 0; j < WA; ++j) ov[j] = 0.0f;
         if (l < nloc) {
             const int g = row0 + l;
-            xr[u] = a.x[g];
-            float ax = diag[l] * xr[u];
+            d = a.A.diag[g];
+            di = d != 0.0f ? 1.0f / d : 1.0f;
+            float xc[WA];
 #pragma unroll
-            for (int j = 0; j < W; ++j) ax += off[j * R + l] * a.x[a.m.ell_col[(size_t)j * C + g]];
+            for (int j = 0; j < W; ++j) {
+                ov[j] = a.A.off[(size_t)j * C + g];
+                const int c = a.m.ell_col[(size_t)j * C + g];
+                const int rk = c / R, lo = c - rk * R;
+                xc[j] = a.x[c];
+                at[u][j] = rk == (int)me ? ub0 + 4u * lo : map_rank(ub + lo, rk);
+                mine = mine && rk == (int)me;
+            }
+            xr[u] = a.x[g];
             const float bi = a.A.rhs[g];
-            const float ri = bi - ax;
+            const float ri = bi - row_product<W>(d, xr[u], ov, xc, false);
             rr_[u] = ri;
-            ub[l] = ri * invd[l];
-            ff_fma(acc[0], ri, ri);
-            ff_fma(acc[2], bi, bi);
+            ur[u] = ri * di;
+            ff_fma(acc[0][u % NA], ri, ri);
+            ff_fma(acc[2][u % NA], bi, bi);
         }
+        ub[l] = ur[u];
+        if constexpr (REG) {
+            dg[u] = d;
+            iv[u] = di;
+#pragma unroll
+            for (int j = 0; j < W; ++j) o[u][j] = ov[j];
+        } else {
+            s_d[u * T + t0] = d;
+            s_i[u * T + t0] = di;
+            if constexpr (W == 4) reinterpret_cast<float4*>(s_o)[u * T + t0] = make_float4(ov[0], ov[1], ov[2], ov[3]);
+            else
+#pragma unroll
+                for (int j = 0; j < W; ++j) s_o[(u * W + j) * T + t0] = ov[j];
+        }
+        if (__all_sync(0xffffffffu, mine)) local |= 1u << u;
     }
     unsigned parity = 0;
     ff red[3];
-    cluster_reduce_tree<3>(acc, red, sbuf, slots, parity, me, cs);
+    cg1m_reduce<T>(acc, red, sbuf, slots, parity, me, cs);
     parity ^= 1u;
     if (t0 == 0) {
         const double rr0 = ff_to_double(red[0]);
@@ -334,57 +431,79 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
             a.stats->rhs_norm = sqrt(ff_to_double(red[2]));
         }
     }
-    __syncthreads();  // the cluster barrier above also published u0 to every CTA
+    __syncthreads();  // the barrier above also published u0 to every CTA
     while (sc.go) {
         const float af = sc.af, bf = sc.bf;
         // (1) s = w + beta s ; p = u + beta p ; x += alpha p ; r -= alpha s ; u = M r
         if (sc.k >= 0) {
 #pragma unroll
-            for (int u = 0; u < RPT; ++u) {
-                const int l = t0 + u * CBS;
-                if (l < nloc) {
-                    const float si = wr[u] + bf * sr[u];
-                    const float pi = ub[l] + bf * pr[u];
-                    xr[u] += af * pi;
-                    const float ri = rr_[u] - af * si;
-                    sr[u] = si;
-                    pr[u] = pi;
-                    rr_[u] = ri;
-                    ub[l] = ri * invd[l];
+            for (int u0 = 0; u0 < RPT; u0 += GR) {
+                if (u0 >= groups * GR) break;
+#pragma unroll
+                for (int u = u0; u < u0 + GR; ++u) {
+                    float di;
+                    if constexpr (REG) di = iv[u];
+                    else di = s_i[u * T + t0];
+                    sr[u] = fmaf(bf, sr[u], wr[u]);
+                    pr[u] = fmaf(bf, pr[u], ur[u]);
+                    xr[u] = fmaf(af, pr[u], xr[u]);
+                    rr_[u] = fmaf(-af, sr[u], rr_[u]);
+                    ur[u] = __fmul_rn(rr_[u], di);
+                    ub[cg1m_row<T>(t0, u)] = ur[u];
                 }
             }
-            cluster_sync_all();  // every CTA's new u, visible to the cluster
+            if (cs > 1) cluster_sync_all();  // every CTA's new u, visible to the cluster
+            else __syncthreads();
         }
-        // (2) w = A u ; r.r ; r.u ; w.u
-        ff acc3[3] = {ff_zero(), ff_zero(), ff_zero()};
+        // (2) w = A u ; r.r ; r.u ; w.u.  The gathers of GR rows are issued before the first is used.
 #pragma unroll
-        for (int u = 0; u < RPT; ++u) {
-            const int l = t0 + u * CBS;
-            if (l < nloc) {
-                const float ui = ub[l];
-                float wi = diag[l] * ui;
-                if (chunk_local[l >> 5]) {  // warp-uniform: every neighbour in this CTA
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-                    for (int j = 0; j < W; ++j) wi += off[j * R + l] * ub[colp[j * R + l] & 0xFFFu];
+            for (int q = 0; q < NA; ++q) acc[i][q] = ff_zero();
+#pragma unroll
+        for (int u0 = 0; u0 < RPT; u0 += GR) {
+            if (u0 >= groups * GR) break;
+            float g[GR][WA];
+#pragma unroll
+            for (int q = 0; q < GR; ++q) {
+                const int u = u0 + q;
+                if ((local >> u) & 1u) {  // warp-uniform: every neighbour in this CTA
+#pragma unroll
+                    for (int j = 0; j < W; ++j) g[q][j] = ld_shared_f32(at[u][j]);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < W; ++j) {
-                        const unsigned cp = colp[j * R + l];
-                        const unsigned rk = cp >> 12;
-                        const unsigned lo = cp & 0xFFFu;
-                        const float uc = rk == me ? ub[lo] : ld_cluster_f32(map_rank(ub + lo, rk));
-                        wi += off[j * R + l] * uc;
+                    for (int j = 0; j < W; ++j) g[q][j] = ld_cluster_f32(at[u][j]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < GR; ++q) {
+                const int u = u0 + q;
+                float ov[WA], d;
+                if constexpr (REG) {
+                    d = dg[u];
+#pragma unroll
+                    for (int j = 0; j < W; ++j) ov[j] = o[u][j];
+                } else {
+                    d = s_d[u * T + t0];
+                    if constexpr (W == 4) {
+                        const float4 v = reinterpret_cast<const float4*>(s_o)[u * T + t0];
+                        ov[0] = v.x; ov[1] = v.y; ov[2] = v.z; ov[3] = v.w;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < W; ++j) ov[j] = s_o[(u * W + j) * T + t0];
                     }
                 }
+                float wi = __fmul_rn(d, ur[u]);
+#pragma unroll
+                for (int j = 0; j < W; ++j) wi = fmaf(ov[j], g[q][j], wi);
                 wr[u] = wi;
-                const float ri = rr_[u];
-                ff_fma(acc3[0], ri, ri);
-                ff_fma(acc3[1], ri, ui);
-                ff_fma(acc3[2], wi, ui);
+                ff_fma(acc[0][u % NA], rr_[u], rr_[u]);
+                ff_fma(acc[1][u % NA], rr_[u], ur[u]);
+                ff_fma(acc[2][u % NA], wi, ur[u]);
             }
         }
         ff d3[3];
-        cluster_reduce_tree<3>(acc3, d3, sbuf, slots, parity, me, cs);
+        cg1m_reduce<T>(acc, d3, sbuf, slots, parity, me, cs);
         parity ^= 1u;
         if (t0 == 0) {
             const ff rr = ff_norm(d3[0]), gamma = ff_norm(d3[1]), delta = ff_norm(d3[2]);
@@ -416,7 +535,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
     }
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
-        const int l = t0 + u * CBS;
+        const int l = cg1m_row<T>(t0, u);
         if (l < nloc) a.x[row0 + l] = xr[u];
     }
     if (me == 0 && t0 == 0) {
@@ -430,8 +549,8 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
 
 // One cluster per case of a device case table, as cg_cluster_batched (krylov_cluster.cu):
 // the same systems, warm starts, refinement mode and stats, the single-reduction CG.
-template <int W, int RPT>
-__global__ void __launch_bounds__(CBS) cg1m_cluster_batched(const wcfd_case* __restrict__ cases, int cs, int refine) {
+template <int W, int RPT, int T>
+__global__ void __launch_bounds__(T, 1) cg1m_cluster_batched(const wcfd_case* __restrict__ cases, int cs, int refine) {
     const wcfd_case& c = cases[blockIdx.x / cs];
     KrylovArgs a = {};
     a.m = c.mesh;
@@ -447,28 +566,31 @@ __global__ void __launch_bounds__(CBS) cg1m_cluster_batched(const wcfd_case* __r
     }
     a.maxiter = c.prm.maxiter;
     a.stats = c.stats + 1;
-    cg1m_cluster_body<W, RPT>(a, (c.mesh.n_cells + cs - 1) / cs);
+    cg1m_cluster_body<W, RPT, T>(a, (c.mesh.n_cells + cs - 1) / cs);
 }
 
-#define WCFD_CG1M_CASE(Wv)                                                      \
-    case Wv * 8 + 1: return (const void*)cg1m_cluster_batched<Wv, 1>;           \
-    case Wv * 8 + 2: return (const void*)cg1m_cluster_batched<Wv, 2>;           \
-    case Wv * 8 + 4: return (const void*)cg1m_cluster_batched<Wv, 4>;
+template <int W>
+static const void* cg1m_pick(int R) {
+    switch (cg1m_capacity(R)) {
+        case 512: return (const void*)cg1m_cluster_batched<W, 2, 256>;
+        case 1024: return (const void*)cg1m_cluster_batched<W, 4, 256>;
+        case 2048: return (const void*)cg1m_cluster_batched<W, 8, 256>;
+        default: return (const void*)cg1m_cluster_batched<W, 8, 512>;
+    }
+}
 
 const void* cg1m_cluster_batched_for(int W, int R) {
-    if (R > 4096) return nullptr;  // 12-bit local index of the packed columns
-    const int rpt = cluster_cg_rpt(R);
-    switch (W * 8 + rpt) {
-        WCFD_CG1M_CASE(0)
-        WCFD_CG1M_CASE(1)
-        WCFD_CG1M_CASE(2)
-        WCFD_CG1M_CASE(3)
-        WCFD_CG1M_CASE(4)
-        WCFD_CG1M_CASE(5)
-        WCFD_CG1M_CASE(6)
+    if (R > 4096) return nullptr;
+    switch (W) {
+        case 0: return cg1m_pick<0>(R);
+        case 1: return cg1m_pick<1>(R);
+        case 2: return cg1m_pick<2>(R);
+        case 3: return cg1m_pick<3>(R);
+        case 4: return cg1m_pick<4>(R);
+        case 5: return cg1m_pick<5>(R);
+        case 6: return cg1m_pick<6>(R);
         default: return nullptr;
     }
 }
-#undef WCFD_CG1M_CASE
 
 }  // namespace wcfd
