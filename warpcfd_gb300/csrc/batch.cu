@@ -122,10 +122,10 @@ const void* batch_cg_kernel(const wcfd_batch_dims& d, int R) {
     return d.cg_variant == 1 ? cg1m_cluster_batched_for(d.ell_width, R) : cg_cluster_batched_for(d.ell_width, R);
 }
 int batch_cg_threads(const wcfd_batch_dims& d, int R) {
-    return d.cg_variant == 1 ? cluster_cg1m_threads(R) : cluster_cg_threads(R, true);
+    return d.cg_variant == 1 ? cluster_cg1m_threads(R) : cluster_cg_threads(R);
 }
 size_t batch_cg_smem(const wcfd_batch_dims& d, int R) {
-    return d.cg_variant == 1 ? cluster_cg1m_smem_bytes(R, d.ell_width) : cluster_cg_smem_bytes(R, d.ell_width, true);
+    return d.cg_variant == 1 ? cluster_cg1m_smem_bytes(R, d.ell_width) : cluster_cg_smem_bytes(R, d.ell_width);
 }
 
 #define BCHECK(what)                                                                               \

@@ -234,8 +234,8 @@ int try_cluster_cg(const wcfd_mesh* m, wcfd_system A, float* x, double atol, int
     if (cs == 0) return -1;
     // the textbook kernel; the single-reduction arrangement when asked for (path 3) and its
     // registers (<= 2 rows per thread) and shared memory allow
-    size_t smem = cluster_cg_smem_bytes(R, W, false);
-    int threads = cluster_cg_threads(R, false);
+    size_t smem = cluster_cg_smem_bytes(R, W);
+    int threads = cluster_cg_threads(R);
     const void* fn = cg_cluster_kernel_for(W, R);
     const size_t smem1 = cluster_cg1_smem_bytes(R, W);
     if (g_krylov_path == 3 && R <= 2 * kClusterBlock && smem1 + 2048 <= (size_t)optin) {

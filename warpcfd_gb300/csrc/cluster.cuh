@@ -22,13 +22,14 @@ __device__ __forceinline__ unsigned cluster_nranks() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The cluster barrier of a reduction: warp 0 (which made the remote slot stores) arrives
-// with release semantics, the other warps arrive relaxed, every thread waits with acquire.
-// Everything the other warps wrote before the CTA's last __syncthreads happens before
-// warp 0's release (the CTA barrier orders it, and the release is cumulative), so the
-// other CTAs see it after their wait; a release by 32 instead of 1,024 threads.
-__device__ __forceinline__ void cluster_sync_warp0_release() {
-    if (threadIdx.x < 32)
+// The cluster barrier of a reduction: the first n warps (which made the remote slot stores)
+// arrive with release semantics, the other warps arrive relaxed, every thread waits with
+// acquire.  Everything the other warps wrote before the CTA's last __syncthreads happens
+// before warp 0's release (the CTA barrier orders it, and the release is cumulative), so the
+// other CTAs see it after their wait; a release by few threads instead of all.
+template <int N>
+__device__ __forceinline__ void cluster_sync_release() {
+    if (threadIdx.x < 32 * N)
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     else
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -104,7 +105,7 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
             if ((unsigned)t < cs) st_cluster_v2f32(map_rank(slots + (parity * NV + i) * 16 + me, t), x.hi, x.lo);
         }
     }
-    cluster_sync_warp0_release();
+    cluster_sync_release<1>();
     if (t < 32) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
@@ -116,60 +117,85 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
     }
 }
 
-// The same sums for CTAs of 256 threads, to every thread (normalised, the same bits): every
-// thread stores its value, warp 0 merges eight each (l, l+32, ..., pairwise), then by butterfly,
-// and stores the CTA total into a slot of every CTA (DSMEM); after the cluster barrier every
-// warp merges the cs <= 16 slots, so that no block barrier and no broadcast follows: the eight
-// warps form the scalars redundantly.  With the caller's four accumulators per thread merged
-// as cluster_reduce_tree merges its quarters (narrow_merge), the sums are those of that tree
-// bit for bit.  (Every warp storing its own total to every CTA, eight times the remote stores:
-// 2,000-2,400 cycles a reduction on 16 CTAs against 1,900.)
-// sbuf: [kClusterSums][256]; slots: [2][kClusterSums][16], double-buffered by `parity`; remote:
-// the address of slots in CTA `lane` (any CTA for lanes past the cluster).
+// Row of thread t's u-th in a CTA of T = 256 or 512 threads, and the number of accumulators it
+// adds its products to (row u to accumulator u % kClusterAcc): chosen so that merging a thread's
+// accumulators (cluster_merge) and then the threads' (below) is the tree of cluster_reduce_tree
+// over 1,024 threads that own the rows t, t + 1024, ... -- the same sums bit for bit whatever
+// T and the rows per thread are, so a case's result does not depend on the kernel that its
+// batch's largest case asks for.
+template <int T>
+__device__ __forceinline__ int cluster_row(int t, int u) {
+    static_assert(T == 256 || T == 512, "the two block sizes");
+    if constexpr (T == 256) return t + 256 * u;
+    else return (t & 255) + ((t >> 8) << 9) + 256 * (u & 1) + 1024 * (u >> 1);
+}
+template <int T>
+constexpr int kClusterAcc = T == 256 ? 4 : 2;
+template <int T>
+__device__ __forceinline__ ff cluster_merge(ff (&acc)[kClusterAcc<T>]) {
+    ff_merge(acc[0], acc[1]);
+    if constexpr (T == 256) {
+        ff_merge(acc[2], acc[3]);
+        ff_merge(acc[0], acc[2]);
+    }
+    return acc[0];
+}
+
+// Sum NV float-float values (cluster_merge of each thread's accumulators) over the CTAs of the
+// cluster, the sums (normalised, the same bits) in every thread.  Warp i merges value i over
+// the CTA's threads (eight or sixteen per lane, pairwise, then by butterfly) and stores the
+// total into a slot of every CTA (DSMEM); the cluster barrier follows.  With eight warps every
+// warp then merges the cs <= 16 slots, so that no block barrier and no broadcast follows (the
+// eight warps form the scalars redundantly); with sixteen, warp i merges value i and a block
+// barrier passes the sums on.  (Every warp storing its own total to every CTA, eight times the
+// remote stores: 2,000-2,400 cycles a reduction on 16 CTAs against 1,900.)
+// sbuf: [kClusterSums][T]; slots: [2][kClusterSums][16], double-buffered by `parity`; remote:
+// the address of slots in CTA `lane`; res: [kClusterSums] (T = 512).
 constexpr int kClusterSums = 3;
-constexpr int kNarrowBlock = 256;
-template <int NV>
-__device__ __forceinline__ void cluster_reduce_narrow(ff (&v)[NV], ff* sbuf, const ff* slots, uint32_t remote,
-                                                      unsigned parity, unsigned me, unsigned cs) {
-    static_assert(NV <= kClusterSums && kNarrowBlock == 256, "eight warps");
-    const int t = threadIdx.x, lane = t & 31;
+template <int NV, int T>
+__device__ __forceinline__ void cluster_reduce_all(ff (&v)[NV], ff* sbuf, const ff* slots, ff* res, uint32_t remote,
+                                                   unsigned parity, unsigned me, unsigned cs) {
+    static_assert(NV <= kClusterSums, "three sums at most");
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
     const unsigned base = parity * (kClusterSums * 16);
 #pragma unroll
-    for (int i = 0; i < NV; ++i) sbuf[i * kNarrowBlock + t] = v[i];
+    for (int i = 0; i < NV; ++i) sbuf[i * T + t] = v[i];
     __syncthreads();
-    if (t < 32) {
-        ff y[NV][8];
+    if (wid < NV) {
+        ff y[8];
 #pragma unroll
-        for (int i = 0; i < NV; ++i)
+        for (int k = 0; k < 8; ++k) y[k] = sbuf[wid * T + 32 * k + lane];
+        if constexpr (T == 512) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) y[i][k] = sbuf[i * kNarrowBlock + 32 * k + t];
+            for (int k = 0; k < 8; ++k) ff_merge(y[k], sbuf[wid * T + 256 + 32 * k + lane]);
+        }
+        ff_tree(y);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) ff_tree(y[i]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) ff_shfl_merge(y[i][0], o);
-        if ((unsigned)t < cs)
-#pragma unroll
-            for (int i = 0; i < NV; ++i)
-                st_cluster_v2f32(remote + (base + i * 16 + me) * (unsigned)sizeof(ff), y[i][0].hi, y[i][0].lo);
+        for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(y[0], o);
+        if ((unsigned)lane < cs)
+            st_cluster_v2f32(remote + (base + wid * 16 + me) * (unsigned)sizeof(ff), y[0].hi, y[0].lo);
     }
-    cluster_sync_warp0_release();
+    cluster_sync_release<NV>();
+    if constexpr (T == 256) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = (unsigned)(lane & 15) < cs ? slots[base + i * 16 + (lane & 15)] : ff_zero();
+        for (int i = 0; i < NV; ++i) v[i] = (unsigned)(lane & 15) < cs ? slots[base + i * 16 + (lane & 15)] : ff_zero();
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1)
+        for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-        for (int i = 0; i < NV; ++i) ff_shfl_merge(v[i], o);
+            for (int i = 0; i < NV; ++i) ff_shfl_merge(v[i], o);
+    } else {
+        if (wid < NV) {
+            ff y = (unsigned)(lane & 15) < cs ? slots[base + wid * 16 + (lane & 15)] : ff_zero();
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) ff_shfl_merge(y, o);
+            if (lane == 0) res[wid] = y;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = res[i];
+    }
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = ff_norm(v[i]);
-}
-// a thread's accumulators of the rows t + 256 (4 m + q), q = 0..3, in acc[q]
-__device__ __forceinline__ ff narrow_merge(ff (&acc)[4]) {
-    ff_merge(acc[0], acc[1]);
-    ff_merge(acc[2], acc[3]);
-    ff_merge(acc[0], acc[2]);
-    return acc[0];
 }
 
 __device__ __forceinline__ float ld_shared_f32(uint32_t addr) {

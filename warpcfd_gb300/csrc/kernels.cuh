@@ -88,10 +88,9 @@ const void* bicgstab_kernel_for(int W);
 const void* cg_cluster_kernel_for(int W, int R);
 const void* cg_cluster_batched_for(int W, int R);
 const void* bicgstab_cluster_batched_for(int W);
-size_t cluster_cg_smem_bytes(int R, int W, bool batched);
-int cluster_cg_threads(int R, bool batched);
+size_t cluster_cg_smem_bytes(int R, int W);
+int cluster_cg_threads(int R);
 int cluster_cg_max_rows(int W, int optin);
-int cluster_cg_rpt(int R);
 const void* cg1_cluster_kernel_for(int W, int R);
 size_t cluster_cg1_smem_bytes(int R, int W);
 // the batched form's single-reduction CG (wcfd_batch_dims.cg_variant = 1), up to 4,096 rows per CTA

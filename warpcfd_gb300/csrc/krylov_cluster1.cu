@@ -267,25 +267,12 @@ size_t cluster_cg1m_smem_bytes(int R, int W) {
     return 4 * (size_t)cap + (cap > 2048 ? (4 * (size_t)W + 8) * cap : 0);
 }
 
-// Row of thread t's u-th in a CTA of T threads, and the accumulator it adds to: chosen so that
-// merging a thread's accumulators and then the threads' (cg1m_reduce) is the tree of
-// cluster_reduce_tree over 1,024 threads that own the rows t, t + 1024, ... -- the same sums bit
-// for bit whatever T and RPT are, so a case's result does not depend on the kernel that its
-// batch's largest case asks for.
-template <int T>
-__device__ __forceinline__ int cg1m_row(int t, int u) {
-    if constexpr (T == 256) return t + 256 * u;
-    else return (t & 255) + ((t >> 8) << 9) + 256 * (u & 1) + 1024 * (u >> 1);
-}
-template <int T>
-constexpr int kCg1mAcc = T == 256 ? 4 : 2;
-
 // Sum three float-float values over the cluster's CTAs, the sums (normalised, the same bits) to
 // thread 0.  acc[i][q]: the accumulators of value i.  Warp i merges value i over the CTA's
 // threads and stores it to every CTA's slots; a cluster of one CTA needs neither DSMEM nor
 // the cluster barrier.  sbuf: [3][T]; slots: [2][3][16], double-buffered by `parity`.
 template <int T>
-__device__ __forceinline__ void cg1m_reduce(ff (&acc)[3][kCg1mAcc<T>], ff (&out)[3], ff* sbuf, ff* slots, unsigned parity,
+__device__ __forceinline__ void cg1m_reduce(ff (&acc)[3][kClusterAcc<T>], ff (&out)[3], ff* sbuf, ff* slots, unsigned parity,
                                             unsigned me, unsigned cs) {
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
     const unsigned base = parity * 48;
@@ -312,7 +299,7 @@ __device__ __forceinline__ void cg1m_reduce(ff (&acc)[3][kCg1mAcc<T>], ff (&out)
         for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(y[0], o);
         if ((unsigned)lane < cs) st_cluster_v2f32(map_rank(slots + base + wid * 16 + me, lane), y[0].hi, y[0].lo);
     }
-    if (cs > 1) cluster_sync_all();
+    if (cs > 1) cluster_sync_release<3>();
     else __syncthreads();
     if (wid == 0) {
 #pragma unroll
@@ -336,7 +323,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         int go, status, k;
     };
     __shared__ Scal sc;
-    constexpr int WA = W > 0 ? W : 1, NA = kCg1mAcc<T>, GR = RPT < 1024 / T ? RPT : 1024 / T;
+    constexpr int WA = W > 0 ? W : 1, NA = kClusterAcc<T>, GR = RPT < 1024 / T ? RPT : 1024 / T;
     constexpr bool REG = kMatrixInRegisters<RPT, T>;
     constexpr int RM = REG ? RPT : 1;
     const int C = a.m.n_cells;
@@ -365,7 +352,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         for (int q = 0; q < NA; ++q) acc[i][q] = ff_zero();
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
-        const int l = cg1m_row<T>(t0, u);
+        const int l = cluster_row<T>(t0, u);
         xr[u] = pr[u] = sr[u] = rr_[u] = wr[u] = ur[u] = 0.0f;
 #pragma unroll
         for (int j = 0; j < W; ++j) at[u][j] = ub0 + 4u * l;
@@ -449,7 +436,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
                     xr[u] = fmaf(af, pr[u], xr[u]);
                     rr_[u] = fmaf(-af, sr[u], rr_[u]);
                     ur[u] = __fmul_rn(rr_[u], di);
-                    ub[cg1m_row<T>(t0, u)] = ur[u];
+                    ub[cluster_row<T>(t0, u)] = ur[u];
                 }
             }
             if (cs > 1) cluster_sync_all();  // every CTA's new u, visible to the cluster
@@ -535,7 +522,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
     }
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
-        const int l = cg1m_row<T>(t0, u);
+        const int l = cluster_row<T>(t0, u);
         if (l < nloc) a.x[row0 + l] = xr[u];
     }
     if (me == 0 && t0 == 0) {
