@@ -231,7 +231,7 @@ class FVM:
     def divFlux(self, arr=None):
         self._need_final()
         if arr is None:
-            arr = torch.zeros(self.num_cells, dtype=self.float_dtype, device=self.device)
+            arr = torch.empty(self.num_cells, dtype=self.float_dtype, device=self.device)
         _lib.call("wcfd_div_flux", ct.byref(self.mesh_struct()), _ptr(self.mass_fluxes), _ptr(arr), _stream())
         return arr
 

@@ -391,7 +391,16 @@ int wcfd_face_pass_flags(const wcfd_mesh* m, wcfd_bc bc, wcfd_state s, uint32_t 
 }
 
 int wcfd_set_boundary_conditions(const wcfd_mesh* m, wcfd_bc bc, wcfd_state s, void* stream) {
-    return wcfd_face_pass_flags(m, bc, s, 0u, 1u, stream);
+    // without the list of boundary faces, the pass over all of them
+    if (!m || !m->boundary_face || m->n_bfaces <= 0) return wcfd_face_pass_flags(m, bc, s, 0u, 1u, stream);
+    int rc = check_mesh(m);
+    if (rc) return rc;
+    RET_IF(!bc.type || !bc.value || !s.cell_values || !s.cell_gradients || !s.face_values || !s.face_gradients ||
+               !s.mass_fluxes,
+           WCFD_ERR_ARGUMENT, "null field");
+    boundary_values_kernel<<<grid_for(m->n_bfaces), kBlock, 0, S(stream)>>>(*m, bc, s);
+    LAUNCH_CHECK("boundary_values_kernel");
+    return WCFD_OK;
 }
 
 int wcfd_face_interpolation(const wcfd_mesh* m, wcfd_bc bc, wcfd_state s, uint32_t mask, int32_t skew,
