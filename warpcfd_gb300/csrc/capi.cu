@@ -582,7 +582,7 @@ int wcfd_assemble_terms(const wcfd_mesh* m, wcfd_system A, const wcfd_term* term
         tl.scale[t] = terms[t].scale;
         tl.cell_based[t] = terms[t].cell_based ? 1 : 0;
     }
-    assemble_terms_kernel<<<grid_for(m->n_cells), kBlock, 0, S(stream)>>>(*m, A, tl);
+    launch_assemble_terms(*m, A, tl, S(stream));
     LAUNCH_CHECK("assemble_terms_kernel");
     return WCFD_OK;
 }

@@ -42,7 +42,7 @@ __global__ void diffusion_weights_kernel(wcfd_mesh m, wcfd_bc bc, wcfd_state s, 
                                          const float* nu_faces, int corrected, int bc_mode, float bc_value, float* w);
 __global__ void ddt_weights_kernel(wcfd_mesh m, wcfd_state s, wcfd_term_fields tf, float dt, float* w);
 __global__ void grad_weights_kernel(wcfd_mesh m, wcfd_state s, int field, float* w);
-__global__ void assemble_terms_kernel(wcfd_mesh m, wcfd_system sys, TermList tl);
+void launch_assemble_terms(const wcfd_mesh& m, const wcfd_system& sys, const TermList& tl, cudaStream_t st);  // ncomp 1 or 3
 __global__ void add_rhs_kernel(int64_t n, float* rhs, const float* a, float scale);
 
 // batched forms over a device case table (blockIdx.y = case)
