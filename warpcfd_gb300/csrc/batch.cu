@@ -128,6 +128,20 @@ size_t batch_cg_smem(const wcfd_batch_dims& d, int R) {
     return d.cg_variant == 1 ? cluster_cg1m_smem_bytes(R, d.ell_width) : cluster_cg_smem_bytes(R, d.ell_width);
 }
 
+// the momentum BiCGSTAB of the batch: everything in shared memory where the largest case's rows per
+// CTA fit
+struct BatchBicg {
+    const void* fn;
+    size_t smem;
+};
+BatchBicg batch_bicg(const wcfd_batch_dims& d, int R) {
+    int dev = 0, optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const bool resident = R <= cluster_bicg_max_rows(d.ell_width, optin);
+    return {bicgstab_cluster_batched_for(d.ell_width, resident), resident ? cluster_bicg_smem_bytes(R, d.ell_width) : 0};
+}
+
 #define BCHECK(what)                                                                               \
     do {                                                                                           \
         const cudaError_t e_ = cudaGetLastError();                                                 \
@@ -148,9 +162,9 @@ extern "C" int wcfd_batch_prepare(const wcfd_batch_dims* dims) {
     if (dims->cg_variant != 0 && dims->cg_variant != 1) return WCFD_ERR_ARGUMENT;
     const int R = (dims->max_cells + cs - 1) / cs;
     const void* cg_fn = batch_cg_kernel(*dims, R);
-    const void* bi_fn = bicgstab_cluster_batched_for(dims->ell_width);
-    if (!cg_fn || !bi_fn) return WCFD_ERR_ARGUMENT;
-    int rc = prepare_cluster(bi_fn, 0);
+    const BatchBicg bi = batch_bicg(*dims, R);
+    if (!cg_fn || !bi.fn) return WCFD_ERR_ARGUMENT;
+    int rc = prepare_cluster(bi.fn, bi.smem);
     if (!rc) rc = prepare_cluster(cg_fn, batch_cg_smem(*dims, R));
     return rc;
 }
@@ -194,8 +208,8 @@ extern "C" int wcfd_batch_simple_iteration(const wcfd_case* cases, int32_t n_cas
         return WCFD_ERR_TOO_LARGE;
     }
     const void* cg_fn = batch_cg_kernel(d, R);
-    const void* bi_fn = bicgstab_cluster_batched_for(d.ell_width);
-    if (!cg_fn || !bi_fn) return WCFD_ERR_ARGUMENT;
+    const BatchBicg bi = batch_bicg(d, R);
+    if (!cg_fn || !bi.fn) return WCFD_ERR_ARGUMENT;
     cudaStream_t st = S(stream);
     NvtxRange step_range("wcfd batched iteration");
     const dim3 gf((d.max_faces + fb - 1) / fb, n_cases), gc((d.max_cells + fb - 1) / fb, n_cases);
@@ -207,9 +221,9 @@ extern "C" int wcfd_batch_simple_iteration(const wcfd_case* cases, int32_t n_cas
     // :102-116
     launch_assemble_batched(false, d.explicit_terms != 0, gc, fb, st, cases);
     BCHECK("momentum_assemble_batched");
-    int csv = cs;
-    void* bargs[] = {(void*)&cases, &csv};
-    int rc = launch_cluster(bi_fn, n_cases, cs, kClusterBlock, 0, st, bargs);
+    int csv = cs, cap = R;
+    void* bargs[] = {(void*)&cases, &csv, &cap};
+    int rc = launch_cluster(bi.fn, n_cases, cs, kBiClusterBlock, bi.smem, st, bargs);
     if (rc) return rc;
     // :118-123
     hbya_batched<<<gc, fb, 0, st>>>(cases);

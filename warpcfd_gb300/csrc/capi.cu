@@ -10,8 +10,8 @@ using namespace wcfd;
 
 // rows per block the grid-cooperative Krylov kernels are sized for (capped at the blocks
 // that can be co-resident)
-#ifndef WCFD_GRID_ROWS_PER_BLOCK
-#define WCFD_GRID_ROWS_PER_BLOCK 1024
+#ifndef WCFD_BICG_ROWS_PER_BLOCK
+#define WCFD_BICG_ROWS_PER_BLOCK 256  // 32,000 rows: 6.5 us an iteration, with 512 7.3, with 128 6.2
 #endif
 #ifndef WCFD_CG_ROWS_PER_BLOCK
 #define WCFD_CG_ROWS_PER_BLOCK 512
@@ -133,9 +133,7 @@ int resident_grid(const void* fn, long long n) {
     return want < cap ? (want < 1 ? 1 : want) : cap;
 }
 
-int launch_krylov(bool cg, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws,
-                  double atol, int maxiter, wcfd_solve_stats* stats, cudaStream_t st, const char* name,
-                  double rtol = 0.0) {
+int check_solve(const wcfd_mesh* m, wcfd_system A, const float* x, wcfd_krylov_ws ws, double atol, int maxiter, const wcfd_solve_stats* stats) {
     int rc = check_mesh(m);
     if (rc) return rc;
     RET_IF(!A.diag || !A.off || !A.rhs || !x || !ws.vec || !ws.partials || !ws.barrier || !stats,
@@ -144,19 +142,39 @@ int launch_krylov(bool cg, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_kry
     RET_IF(reinterpret_cast<uintptr_t>(ws.partials) % 16 != 0, WCFD_ERR_ARGUMENT,
            "Krylov workspace: partials must be 16-byte aligned");
     RET_IF(maxiter < 0 || !(atol >= 0.0), WCFD_ERR_ARGUMENT, "bad atol or maxiter");
+    return WCFD_OK;
+}
+
+int launch_krylov(bool cg, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws,
+                  double atol, int maxiter, wcfd_solve_stats* stats, cudaStream_t st, const char* name,
+                  double rtol = 0.0) {
+    int rc = check_solve(m, A, x, ws, atol, maxiter, stats);
+    if (rc) return rc;
     // rows per block, then the kernel for them (a CG kernel's limits do not depend on it)
     const int sms_cap = coop_limits(barrier_check_kernel_ptr(), kSolverBlock, false).blocks;
     LAUNCH_CHECK("occupancy query");
-    const int per_block = cg ? WCFD_CG_ROWS_PER_BLOCK : WCFD_GRID_ROWS_PER_BLOCK;
+    const int per_block = cg ? WCFD_CG_ROWS_PER_BLOCK : WCFD_BICG_ROWS_PER_BLOCK;
     long long want = ((long long)m->n_cells + per_block - 1) / per_block;
     int grid = (int)(want < sms_cap ? want : sms_cap);
     if (grid < 1) grid = 1;
-    const CgKernel ck = cg ? cg_kernel_for(m->ell_width, (int)(((long long)m->n_cells + grid - 1) / grid)) : CgKernel{nullptr, 0};
-    const void* fn = cg ? ck.fn : bicgstab_kernel_for(m->ell_width);
-    RET_IF(!fn, WCFD_ERR_ARGUMENT, "no solver kernel for this off-diagonal width");
-    const int threads = cg ? kCgBlock : kSolverBlock, chunk = ck.chunk;
-    const CoopLimits lim = coop_limits(fn, threads, cg);
+    int rows = (int)(((long long)m->n_cells + grid - 1) / grid);
+    CgKernel ck = cg ? cg_kernel_for(m->ell_width, rows) : CgKernel{bicgstab_kernel_for(m->ell_width, true), 32};
+    RET_IF(!ck.fn, WCFD_ERR_ARGUMENT, "no solver kernel for this off-diagonal width");
+    const int chunk = ck.chunk;
+    CoopLimits lim = coop_limits(ck.fn, kCgBlock, true);
     LAUNCH_CHECK("occupancy query");
+    rows = (rows + (chunk - 1)) / chunk * chunk;
+    size_t smem = 0;
+    if (!cg) {
+        // the resident form while a block's rows fit its shared memory
+        smem = bicgstab_row_bytes(m->ell_width) * rows;
+        if (smem > lim.smem) {
+            smem = 0;
+            ck.fn = bicgstab_kernel_for(m->ell_width, false);
+            lim = coop_limits(ck.fn, kCgBlock, false);
+            LAUNCH_CHECK("occupancy query");
+        }
+    }
     RET_IF(lim.blocks < grid, WCFD_ERR_CUDA, "solver kernel cannot be resident");
     if (cudaMemsetAsync(ws.partials, 0, kGridCtlBytes, st) != cudaSuccess)
         return set_error(WCFD_ERR_CUDA, "barrier reset failed");
@@ -170,14 +188,12 @@ int launch_krylov(bool cg, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_kry
     a.rtol2 = rtol * rtol;
     a.maxiter = maxiter;
     a.stats = stats;
-    size_t smem = 0;
+    a.rows = rows;
+    grid = (int)(((long long)m->n_cells + rows - 1) / rows);
     if (cg) {
         // contiguous rows per block; shared memory goes to the column offsets first (16 or 32
         // bytes per chunk), then to r, q and x (12 bytes a row for the 28 they move an
         // iteration), then to 1/diag (4 for 4)
-        const long long rows = (((long long)m->n_cells + grid - 1) / grid + (chunk - 1)) / chunk * chunk;
-        a.rows = (int)rows;
-        grid = (int)((m->n_cells + rows - 1) / rows);
         size_t left = lim.smem;
         auto take = [&](size_t per_chunk, int most) {  // rows (a multiple of chunk)
             const size_t fit = per_chunk ? left / per_chunk * chunk : (size_t)most;
@@ -192,7 +208,7 @@ int launch_krylov(bool cg, const wcfd_mesh* m, wcfd_system A, float* x, wcfd_kry
     }
     void* args[] = {&a};
     const cudaError_t e =
-        cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, st);
+        cudaLaunchCooperativeKernel(ck.fn, dim3(grid), dim3(kCgBlock), args, smem, st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s", name, cudaGetErrorString(e));
@@ -211,38 +227,12 @@ int g_krylov_path = 0;  // 0 automatic, 1 grid-cooperative only, 2 cluster-resid
 #define WCFD_CLUSTER_ROW_CAP 512
 #endif
 
-// Cluster-resident CG when the system fits in the shared memory of one cluster of up to
-// 16 CTAs; returns -1 (caller falls back to the grid-cooperative kernel) otherwise.
-int try_cluster_cg(const wcfd_mesh* m, wcfd_system A, float* x, double atol, int maxiter,
-                   wcfd_solve_stats* stats, cudaStream_t st, double rtol = 0.0) {
-    if (g_krylov_path == 1) return -1;
-    const int C = m->n_cells, W = m->ell_width;
+// Launch a solve on one cluster of cs CTAs of R rows; -1 when it cannot be scheduled.
+int launch_cluster_solve(const void* fn, int cs, int threads, size_t smem, const wcfd_mesh* m, wcfd_system A, float* x, float* vec,
+                         double atol, double rtol, int maxiter, wcfd_solve_stats* stats, cudaStream_t st, int R, const char* name) {
+    const int C = m->n_cells;
     int dev = 0;
     cudaGetDevice(&dev);
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const int rmax = cluster_cg_max_rows(W, optin);
-    int cs = 0, R = 0;
-    for (int c = 1; c <= 16; c *= 2) {
-        const long long r = (C + c - 1) / c;
-        if (r <= rmax && (r <= WCFD_CLUSTER_ROW_CAP || c == 16)) {
-            cs = c;
-            R = (int)r;
-            break;
-        }
-    }
-    if (cs == 0) return -1;
-    // the textbook kernel; the single-reduction arrangement when asked for (path 3) and its
-    // registers (<= 2 rows per thread) and shared memory allow
-    size_t smem = cluster_cg_smem_bytes(R, W);
-    int threads = cluster_cg_threads(R);
-    const void* fn = cg_cluster_kernel_for(W, R);
-    const size_t smem1 = cluster_cg1_smem_bytes(R, W);
-    if (g_krylov_path == 3 && R <= 2 * kClusterBlock && smem1 + 2048 <= (size_t)optin) {
-        fn = cg1_cluster_kernel_for(W, R);
-        smem = smem1;
-        threads = kClusterBlock;
-    }
     if (!fn) return -1;
     static std::mutex mu;
     struct SetA { const void* fn; int dev; size_t bytes; };
@@ -297,6 +287,7 @@ int try_cluster_cg(const wcfd_mesh* m, wcfd_system A, float* x, double atol, int
     a.m = *m;
     a.A = A;
     a.x = x;
+    a.ws = vec;
     a.atol2 = atol * atol;
     a.rtol2 = rtol * rtol;
     a.maxiter = maxiter;
@@ -305,10 +296,68 @@ int try_cluster_cg(const wcfd_mesh* m, wcfd_system A, float* x, double atol, int
     const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        std::snprintf(g_last_error, sizeof(g_last_error), "cg_cluster_kernel: %s", cudaGetErrorString(e));
+        std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s", name, cudaGetErrorString(e));
         return WCFD_ERR_CUDA;
     }
     return WCFD_OK;
+}
+
+// Cluster-resident CG when the system fits in the shared memory of one cluster of up to
+// 16 CTAs; returns -1 (caller falls back to the grid-cooperative kernel) otherwise.
+int try_cluster_cg(const wcfd_mesh* m, wcfd_system A, float* x, double atol, int maxiter,
+                   wcfd_solve_stats* stats, cudaStream_t st, double rtol = 0.0) {
+    if (g_krylov_path == 1) return -1;
+    const int C = m->n_cells, W = m->ell_width;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const int rmax = cluster_cg_max_rows(W, optin);
+    int cs = 0, R = 0;
+    for (int c = 1; c <= 16; c *= 2) {
+        const long long r = (C + c - 1) / c;
+        if (r <= rmax && (r <= WCFD_CLUSTER_ROW_CAP || c == 16)) {
+            cs = c;
+            R = (int)r;
+            break;
+        }
+    }
+    if (cs == 0) return -1;
+    // the textbook kernel; the single-reduction arrangement when asked for (path 3) and its
+    // registers (<= 2 rows per thread) and shared memory allow
+    size_t smem = cluster_cg_smem_bytes(R, W);
+    int threads = cluster_cg_threads(R);
+    const void* fn = cg_cluster_kernel_for(W, R);
+    const size_t smem1 = cluster_cg1_smem_bytes(R, W);
+    if (g_krylov_path == 3 && R <= 2 * kClusterBlock && smem1 + 2048 <= (size_t)optin) {
+        fn = cg1_cluster_kernel_for(W, R);
+        smem = smem1;
+        threads = kClusterBlock;
+    }
+    return launch_cluster_solve(fn, cs, threads, smem, m, A, x, nullptr, atol, rtol, maxiter, stats, st, R, "cg_cluster_kernel");
+}
+
+// rows per CTA that the cluster BiCGSTAB aims at: 4,096 rows on 16 CTAs 2.86 us an iteration, on 8 3.38
+constexpr int kBicgClusterRows = 256;
+
+// Cluster-resident BiCGSTAB under the same terms: up to 16 CTAs of about 1,000 rows.  With more rows
+// the grid kernel's 152 SMs outweigh its dearer barriers (4,096 rows: 2.9 us an iteration here, 5.8
+// there; 32,000 rows there 6.2).
+int try_cluster_bicgstab(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws, double atol, int maxiter,
+                         wcfd_solve_stats* stats, cudaStream_t st, double rtol) {
+    if (g_krylov_path == 1) return -1;
+    const int rc = check_solve(m, A, x, ws, atol, maxiter, stats);
+    if (rc) return rc;
+    int dev = 0, optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const int C = m->n_cells, W = m->ell_width;
+    int cs = 1;
+    while (cs < 16 && (C + cs - 1) / cs > kBicgClusterRows) cs *= 2;
+    const int R = (C + cs - 1) / cs;
+    if (R > cluster_bicg_max_rows(W, optin)) return -1;
+    return launch_cluster_solve(bicgstab_cluster_kernel_for(W), cs, kBiClusterBlock, cluster_bicg_smem_bytes(R, W), m, A, x,
+                                ws.vec, atol, rtol, maxiter, stats, st, R, "bicgstab_cluster_kernel");
 }
 
 }  // namespace
@@ -661,6 +710,8 @@ static int bicgstab_solve(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_kryl
                           int32_t maxiter, wcfd_solve_stats* stats, void* stream) {
     RET_IF(A.ncomp != 3, WCFD_ERR_ARGUMENT, "bicgstab solves the 3-component momentum system (ncomp 3)");
     RET_IF(!(rtol >= 0.0), WCFD_ERR_ARGUMENT, "bad rtol");
+    const int rc = try_cluster_bicgstab(m, A, x, ws, atol, maxiter, stats, S(stream), rtol);
+    if (rc != -1) return rc;
     return launch_krylov(false, m, A, x, ws, atol, maxiter, stats, S(stream),
                          "bicgstab_kernel", rtol);
 }

@@ -184,6 +184,22 @@ __device__ __forceinline__ float row_product(float d, float p, const float (&o)[
     return q;
 }
 
+// Columns of row i, slot by slot: from the int16 offsets (wcfd_mesh.ell_dcol) when the mesh has
+// them (half the bytes), else the int32 columns.  Every load is issued before the first use.
+template <int W>
+__device__ __forceinline__ void ell_columns(int (&c)[W > 0 ? W : 1], const int* __restrict__ col,
+                                            const int16_t* __restrict__ dcol, int C, int i) {
+    if (dcol) {
+#pragma unroll
+        for (int j = 0; j < W; ++j) c[j] = __ldcs(dcol + (size_t)j * C + i);
+#pragma unroll
+        for (int j = 0; j < W; ++j) c[j] += i;
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) c[j] = __ldcs(col + (size_t)j * C + i);
+    }
+}
+
 // Block total of NV float-float accumulators, still as float-float (the same bits in every
 // thread).  Warps merge by butterfly shuffles, then warp 0 merges the warp totals; no fp64
 // instruction is issued (a full-warp fp64 instruction is expensive on GB300).

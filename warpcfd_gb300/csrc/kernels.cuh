@@ -85,10 +85,15 @@ struct CgKernel {
 CgKernel cg_kernel_for(int W, int rows);
 size_t cg_chunk_bytes(int W);  // shared memory of a chunk's column offsets
 const void* barrier_check_kernel_ptr();
-const void* bicgstab_kernel_for(int W);
+const void* bicgstab_kernel_for(int W, bool resident);
+size_t bicgstab_row_bytes(int W);  // shared memory of a row of the resident form
 const void* cg_cluster_kernel_for(int W, int R);
 const void* cg_cluster_batched_for(int W, int R);
-const void* bicgstab_cluster_batched_for(int W);
+constexpr int kBiClusterBlock = 512;
+const void* bicgstab_cluster_kernel_for(int W);
+const void* bicgstab_cluster_batched_for(int W, bool resident);
+size_t cluster_bicg_smem_bytes(int R, int W);
+int cluster_bicg_max_rows(int W, int optin);
 size_t cluster_cg_smem_bytes(int R, int W);
 int cluster_cg_threads(int R);
 int cluster_cg_max_rows(int W, int optin);

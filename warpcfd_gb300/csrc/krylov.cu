@@ -17,13 +17,14 @@
 // through shared memory behind its last block barrier: GB300
 // runs fp64 at about 1/64 of its fp32 rate (a dependent fp64 division costs about 600
 // cycles), and every thread of the grid waits for these few operations.
+#include "bicgstab.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 
 namespace wcfd {
 
-constexpr int BS = kSolverBlock;  // threads of the BiCGSTAB
-constexpr int CGB = kCgBlock;     // threads of the CG
+constexpr int BS = kSolverBlock;  // threads of the barrier check
+constexpr int CGB = kCgBlock;     // threads of the CG and the BiCGSTAB
 
 __device__ __forceinline__ float jacobi(float d) { return d != 0.0f ? 1.0f / d : 1.0f; }
 
@@ -70,50 +71,6 @@ __device__ void write_stats(const KrylovArgs& a, const KScalars& sc) {
         a.stats->iterations = sc.k;
         a.stats->status = st;
         a.stats->residual = sqrt(ff_to_double(sc.rr));
-    }
-}
-
-// L2 prefetch of the matrix lines that a warp's rows use `ahead` grid-stride trips of one
-// row later: lane l < 2 W takes slab l (columns, then coefficients) and prefetches the
-// lines of the warp's first and last row there (one line when the 32 rows are 128-byte
-// aligned).  Nothing waits on a prefetch and no register is held.  Used by the BiCGSTAB,
-// whose vectors (nine 3C arrays) exceed L2 anyway, where it takes a DRAM round trip out of
-// each trip of the SpMV passes (0.374 -> 0.338 ms per 128^3 momentum solve).  The grid CG
-// keeps its vectors in L2 and reads the matrix evict-first; every prefetch variant tried
-// there (per line at normal priority, or a bulk prefetch of each block's 4 KB slabs with
-// the evict-first policy, 1 to 5 trips ahead) made its iteration slower (35.4 us ->
-// 41-47 us on 128^3).
-template <int W>
-__device__ __forceinline__ void prefetch_matrix_lines(const int* col, const float* off, int C, int stride, int i,
-                                                      int ahead) {
-    if constexpr (W > 0) {
-        const int lane = threadIdx.x & 31;
-        if (lane < 2 * W) {
-            const long long rb = (long long)i - lane + (long long)ahead * stride;
-            if (rb < C) {
-                const long long rl = rb + 31 < C ? rb + 31 : C - 1;
-                const char* base = lane < W ? reinterpret_cast<const char*>(col + (size_t)lane * C)
-                                            : reinterpret_cast<const char*>(off + (size_t)(lane - W) * C);
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)rb * 4));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)rl * 4));
-            }
-        }
-    }
-}
-
-// Columns of row i, slot by slot: from the int16 offsets (wcfd_mesh.ell_dcol) when the mesh has
-// them (half the bytes), else the int32 columns.  Every load is issued before the first use.
-template <int W>
-__device__ __forceinline__ void ell_columns(int (&c)[W > 0 ? W : 1], const int* __restrict__ col,
-                                            const int16_t* __restrict__ dcol, int C, int i) {
-    if (dcol) {
-#pragma unroll
-        for (int j = 0; j < W; ++j) c[j] = __ldcs(dcol + (size_t)j * C + i);
-#pragma unroll
-        for (int j = 0; j < W; ++j) c[j] += i;
-    } else {
-#pragma unroll
-        for (int j = 0; j < W; ++j) c[j] = __ldcs(col + (size_t)j * C + i);
     }
 }
 
@@ -392,205 +349,30 @@ __global__ void __launch_bounds__(CGB, 1) cg_kernel(KrylovArgs a) {
     write_stats(a, sc);
 }
 
-// Right-preconditioned (Jacobi) BiCGSTAB on the 3-component momentum system
-// (interleaved rows 3c+o, shared off-diagonals).
-// Workspace (3C floats each): r, r0, pA, pB, vA, vB, t, s, invd.
-template <int W>
-__global__ void __launch_bounds__(BS) bicgstab_kernel(KrylovArgs a) {
-    __shared__ KScalars sc;
-    __shared__ ff sbuf[2 * BS / 2];
-    const int C = a.m.n_cells;
-    const size_t n3 = 3 * (size_t)C;
-    float* r = a.ws;
-    float* r0 = a.ws + n3;
-    float* pbuf[2] = {a.ws + 2 * n3, a.ws + 3 * n3};
-    float* vbuf[2] = {a.ws + 4 * n3, a.ws + 5 * n3};
-    float* t = a.ws + 6 * n3;
-    float* s = a.ws + 7 * n3;
-    float* invd = a.ws + 8 * n3;
-    const float* __restrict__ b = a.A.rhs;
-    const float* __restrict__ diag = a.A.diag;
-    const float* __restrict__ off = a.A.off;
-    const int* __restrict__ col = a.m.ell_col;
-    float* x = a.x;
-    constexpr int WA = W > 0 ? W : 1;
-    const bool in_place = slot_bits(a.m) != 0u;
-    const int stride = gridDim.x * BS;
-    const int i0 = blockIdx.x * BS + threadIdx.x;
-    unsigned phase = 0;
-    if (threadIdx.x == 0) {
-        sc.k = 0;
-        sc.status = WCFD_OK;
-    }
-
-    // r = b - A x ; r0 = r ; p = r ; v = 0 ; rr ; rho = r0.r = rr ; bb = b.b
-    ff acc[2] = {ff_zero(), ff_zero()};
-    for (int i = i0; i < C; i += stride) {
-        float ax[3], v[WA], g[3][WA];
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            v[j] = __ldcs(off + (size_t)j * C + i);
-            const int c = __ldcs(col + (size_t)j * C + i);
-#pragma unroll
-            for (int o = 0; o < 3; ++o) g[o][j] = x[3 * (size_t)c + o];
-        }
-#pragma unroll
-        for (int o = 0; o < 3; ++o)
-            ax[o] = row_product<W>(diag[3 * (size_t)i + o], x[3 * (size_t)i + o], v, g[o], in_place);
-#pragma unroll
-        for (int o = 0; o < 3; ++o) {
-            const size_t q = 3 * (size_t)i + o;
-            const float ri = b[q] - ax[o];
-            r[q] = ri;
-            r0[q] = ri;
-            pbuf[0][q] = ri;
-            vbuf[0][q] = 0.0f;
-            invd[q] = jacobi(diag[q]);
-            ff_fma(acc[0], ri, ri);
-            ff_fma(acc[1], b[q], b[q]);
-        }
-    }
-    REDUCE(2, acc, [&](const ff* v) {
-        if (threadIdx.x != 0) return;
-        init_scalars(a, sc, v[0]);
-        sc.rho = v[0];
-        sc.bf = 0.0f;  // the first direction is r itself
-        sc.of = 0.0f;
-        if (blockIdx.x == 0) a.stats->rhs_norm = sqrt(ff_to_double(v[1]));
-    });
-    int cur = 0;
-    while (sc.go) {
-        const float bf = sc.bf, of0 = sc.of;
-        const float* po = pbuf[cur];  // written by other blocks in this launch: no restrict
-        const float* vo = vbuf[cur];
-        float* pn = pbuf[cur ^ 1];
-        float* vn = vbuf[cur ^ 1];
-        // p = r + beta (p - omega v) ; v = A (M p) ; r0.v
-        ff accv[1] = {ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-            prefetch_matrix_lines<W>(col, off, C, stride, i, 1);
-            float pi[3], vi[3], v[WA], g[3][WA];
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                pi[o] = r[q] + bf * (po[q] - of0 * vo[q]);
-            }
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                v[j] = __ldcs(off + (size_t)j * C + i);
-                const int c = __ldcs(col + (size_t)j * C + i);
-#pragma unroll
-                for (int o = 0; o < 3; ++o) {
-                    const size_t q = 3 * (size_t)c + o;
-                    const float pc = r[q] + bf * (po[q] - of0 * vo[q]);
-                    g[o][j] = pc * invd[q];
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                vi[o] = row_product<W>(diag[q], pi[o] * invd[q], v, g[o], in_place);
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                pn[q] = pi[o];
-                vn[q] = vi[o];
-                ff_fma(accv[0], r0[q], vi[o]);
-            }
-        }
-        REDUCE(1, accv, [&](const ff* r0v) {
-            if (threadIdx.x != 0) return;
-            if (r0v[0].hi == 0.0f) {
-                sc.status = WCFD_KRYLOV_BREAKDOWN;
-                sc.go = 0;
-            } else {
-                sc.alpha = ff_div(sc.rho, r0v[0]);
-                sc.af = ff_to_float(sc.alpha);
-            }
-        });
-        if (!sc.go) break;
-        const float af = sc.af;
-        // s = r - alpha v ; x += alpha M p ; t = A (M s) ; t.t ; t.s
-        ff acct[2] = {ff_zero(), ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-            prefetch_matrix_lines<W>(col, off, C, stride, i, 1);
-            float si[3], ti[3], v[WA], g[3][WA];
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                v[j] = __ldcs(off + (size_t)j * C + i);
-                const int c = __ldcs(col + (size_t)j * C + i);
-#pragma unroll
-                for (int o = 0; o < 3; ++o) {
-                    const size_t q = 3 * (size_t)c + o;
-                    const float scv = r[q] - af * vn[q];
-                    g[o][j] = scv * invd[q];
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                si[o] = r[q] - af * vn[q];
-                ti[o] = row_product<W>(diag[q], si[o] * invd[q], v, g[o], in_place);
-                x[q] += af * (pn[q] * invd[q]);
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                s[q] = si[o];
-                t[q] = ti[o];
-                ff_fma(acct[0], ti[o], ti[o]);
-                ff_fma(acct[1], ti[o], si[o]);
-            }
-        }
-        REDUCE(2, acct, [&](const ff* ts) {
-            if (threadIdx.x != 0) return;
-            sc.omega = ts[0].hi != 0.0f ? ff_div(ts[1], ts[0]) : ff_zero();
-            sc.of = ff_to_float(sc.omega);
-        });
-        const float of = sc.of;
-        // x += omega M s ; r = s - omega t ; r.r ; r0.r -- every load of the row issued
-        // before its first store (x and r may alias the others as far as the compiler
-        // knows), components accumulated in order
-        ff accr[2] = {ff_zero(), ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-            float sv[3], dv[3], xv[3], tv[3], rv0[3];
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                sv[o] = s[q];
-                dv[o] = invd[q];
-                xv[o] = x[q];
-                tv[o] = t[q];
-                rv0[o] = r0[q];
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                x[q] = xv[o] + of * (sv[o] * dv[o]);
-                const float ri = sv[o] - of * tv[o];
-                r[q] = ri;
-                ff_fma(accr[0], ri, ri);
-                ff_fma(accr[1], rv0[o], ri);
-            }
-        }
-        REDUCE(2, accr, [&](const ff* rr2) {
-            if (threadIdx.x != 0) return;
-            sc.rr = rr2[0];
-            sc.k += 1;
-            if (sc.omega.hi == 0.0f || sc.rho.hi == 0.0f) {
-                sc.status = WCFD_KRYLOV_BREAKDOWN;
-                sc.go = 0;
-            } else {
-                sc.bf = ff_to_float(ff_mul(ff_div(rr2[1], sc.rho), ff_div(sc.alpha, sc.omega)));
-                sc.rho = rr2[1];
-                sc.go = (sc.k < a.maxiter && ff_gt(sc.rr, sc.thr2));
-            }
-        });
-        cur ^= 1;
-    }
-    write_stats(a, sc);
+// BiCGSTAB (bicgstab.cuh) over the grid, a.rows contiguous rows a block; RES: with the rows' own
+// data in shared memory.
+template <int W, bool RES>
+__global__ void __launch_bounds__(kCgBlock, 1) bicgstab_kernel(KrylovArgs a) {
+    extern __shared__ __align__(16) float own[];
+    __shared__ BiScalars sc;
+    __shared__ ff sbuf[kCgBlock];
+    const int C = a.m.n_cells, row0 = (int)blockIdx.x * a.rows;
+    const BiSystem sys{a.A.diag, a.A.off, a.A.rhs, a.m.ell_col, a.m.ell_dcol, a.x, C, a.maxiter, slot_bits(a.m) != 0u, a.atol2, a.rtol2, a.stats};
+    BiGlobal<kCgBlock, false> net(a.ws, C, row0);
+    net.g = a.g;
+    net.sbuf = sbuf;
+    if (!bicgstab_body<W, kCgBlock, RES>(sys, net, sc, own, a.rows, row0, max(0, min(a.rows, C - row0)), blockIdx.x == 0))
+        fail_stats(a, sc.k);
 }
+const void* bicgstab_kernel_for(int W, bool resident) {
+#define WCFD_BI(w) case w: return resident ? (const void*)bicgstab_kernel<w, true> : (const void*)bicgstab_kernel<w, false>;
+    switch (W) {
+        WCFD_BI(0) WCFD_BI(1) WCFD_BI(2) WCFD_BI(3) WCFD_BI(4) WCFD_BI(5) WCFD_BI(6)
+        default: return nullptr;
+    }
+#undef WCFD_BI
+}
+size_t bicgstab_row_bytes(int W) { return sizeof(float) * (kBiPlanes + 2 * (size_t)W); }
 
 // ---------------------------------------------------------------------------------
 // fp64 iterative refinement of a scalar solve (the precision form of the pressure solve):
@@ -677,18 +459,6 @@ const void* cg_kernel_pick(int W) {
     }
 }
 
-const void* bicgstab_kernel_for(int W) {
-    switch (W) {
-        case 0: return (const void*)bicgstab_kernel<0>;
-        case 1: return (const void*)bicgstab_kernel<1>;
-        case 2: return (const void*)bicgstab_kernel<2>;
-        case 3: return (const void*)bicgstab_kernel<3>;
-        case 4: return (const void*)bicgstab_kernel<4>;
-        case 5: return (const void*)bicgstab_kernel<5>;
-        case 6: return (const void*)bicgstab_kernel<6>;
-        default: return nullptr;
-    }
-}
 
 size_t cg_chunk_bytes(int W) { return W > 4 ? sizeof(ChunkCols<5>) : W > 0 ? sizeof(ChunkCols<4>) : 0; }
 

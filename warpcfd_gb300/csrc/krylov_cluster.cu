@@ -22,6 +22,7 @@
 // 3.74 (the grid kernel: 4.59).
 // The arithmetic is that of cg_kernel (krylov.cu): the same Jacobi-preconditioned CG with
 // fp64-accurate dot products and the same stop test.
+#include "bicgstab.cuh"
 #include "cluster.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -271,238 +272,55 @@ __global__ void __launch_bounds__(T, 1) cg_cluster_batched(const wcfd_case* __re
     cg_cluster_body<W, RPT, T>(a, (c.mesh.n_cells + cs - 1) / cs);
 }
 
-// BiCGSTAB on one case per cluster, for the batched form: the momentum system of the
-// case (interleaved 3C rows, shared off-diagonals) with its vectors in global memory
-// (the case's workspace: r, r0, pA, pB, vA, vB, t, s, invd), rows spread over the cluster's
-// CTAs, hardware cluster barriers and the DSMEM all-reduce.  Values written by another CTA
-// during the solve are read through L2 (ld.cg).  Same algorithm and arithmetic as
-// bicgstab_kernel (krylov.cu).
-template <int W>
-__device__ __forceinline__ void bicgstab_cluster_body(const wcfd_case& cse) {
-    __shared__ ff slots[2 * 3 * 16];
-    __shared__ ff sbuf[2 * CBS];
-    struct Scal {
-        ff rr, rho, alpha, omega, thr2;
-        float af, bf, of;
-        int go, status, k;
+// BiCGSTAB (bicgstab.cuh) over the CTAs of one cluster.  SMEM: records in the CTAs' shared memory
+// with the rows' own data, up to about 1,000 rows a CTA; else records in the case's workspace.
+template <int W, bool SMEM>
+__device__ __forceinline__ void bicgstab_cluster_body(const BiSystem& sys, float* ws, int R, int cap) {
+    constexpr int T = kBiClusterBlock;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ BiScalars sc;
+    __shared__ ff slots[2 * kClusterSums * 16], sbuf[2 * T], res[kClusterSums];
+    const unsigned me = cluster_rank(), cs = cluster_nranks();
+    const int row0 = (int)me * R, nloc = max(0, min(R, sys.C - row0));
+    float4* records = reinterpret_cast<float4*>(smem);
+    auto run = [&](auto& net, float* own) {
+        net.sbuf = sbuf;
+        net.slots = slots;
+        net.res = res;
+        net.me = me;
+        net.cs = cs;
+        net.remote = map_rank(slots, min((unsigned)(threadIdx.x & 31), cs - 1));
+        bicgstab_body<W, T, SMEM>(sys, net, sc, own, cap, row0, nloc, me == 0);
     };
-    __shared__ Scal sc;
-    const unsigned me = cluster_rank();
-    const unsigned cs = cluster_nranks();
-    const int C = cse.mesh.n_cells;
-    const size_t n3 = 3 * (size_t)C;
-    float* ws = cse.ws_u.vec;
-    float* r = ws;
-    float* r0 = ws + n3;
-    float* pbuf[2] = {ws + 2 * n3, ws + 3 * n3};
-    float* vbuf[2] = {ws + 4 * n3, ws + 5 * n3};
-    float* t = ws + 6 * n3;
-    float* s = ws + 7 * n3;
-    float* invd = ws + 8 * n3;
-    const float* __restrict__ b = cse.mom.rhs;
-    const float* __restrict__ diag = cse.mom.diag;
-    const float* __restrict__ off = cse.mom.off;
-    const int* __restrict__ col = cse.mesh.ell_col;
-    float* x = cse.hbya;
-    const double atol2 = cse.prm.atol_u * cse.prm.atol_u;
-    const double rtol2 = cse.prm.rtol_u * cse.prm.rtol_u;
-    const int maxiter = cse.prm.maxiter;
-    const int stride = (int)cs * CBS;
-    const int i0 = (int)me * CBS + threadIdx.x;
-    unsigned parity = 0;
-
-    ff acc[2] = {ff_zero(), ff_zero()};
-    for (int i = i0; i < C; i += stride) {
-        float ax[3];
-#pragma unroll
-        for (int o = 0; o < 3; ++o) ax[o] = diag[3 * (size_t)i + o] * x[3 * (size_t)i + o];
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            const float v = off[(size_t)j * C + i];
-            const int c = col[(size_t)j * C + i];
-#pragma unroll
-            for (int o = 0; o < 3; ++o) ax[o] += v * x[3 * (size_t)c + o];
-        }
-#pragma unroll
-        for (int o = 0; o < 3; ++o) {
-            const size_t q = 3 * (size_t)i + o;
-            const float ri = b[q] - ax[o];
-            r[q] = ri;
-            r0[q] = ri;
-            pbuf[0][q] = ri;
-            vbuf[0][q] = 0.0f;
-            invd[q] = diag[q] != 0.0f ? 1.0f / diag[q] : 1.0f;
-            ff_fma(acc[0], ri, ri);
-            ff_fma(acc[1], b[q], b[q]);
-        }
-    }
-    ff red[2];
-    cluster_reduce_tree<2>(acc, red, sbuf, slots, parity, me, cs);
-    parity ^= 1u;
-    if (threadIdx.x == 0) {
-        const double rr0 = ff_to_double(red[0]);
-        sc.rr = ff_norm(red[0]);
-        sc.rho = sc.rr;
-        sc.thr2 = ff_norm(ff_from_double(fmax(atol2, rtol2 * rr0)));
-        sc.bf = 0.0f;
-        sc.of = 0.0f;
-        sc.k = 0;
-        sc.status = WCFD_OK;
-        sc.go = (0 < maxiter && ff_gt(sc.rr, sc.thr2));
-        if (me == 0) {
-            cse.stats[0].initial_residual = sqrt(rr0);
-            cse.stats[0].rhs_norm = sqrt(ff_to_double(red[1]));
-        }
-    }
-    __syncthreads();
-    int cur = 0;
-    while (sc.go) {
-        const float bf = sc.bf, of0 = sc.of;
-        const float* po = pbuf[cur];
-        const float* vo = vbuf[cur];
-        float* pn = pbuf[cur ^ 1];
-        float* vn = vbuf[cur ^ 1];
-        ff accv[1] = {ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-            float pi[3], vi[3];
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                pi[o] = __ldcg(r + q) + bf * (__ldcg(po + q) - of0 * __ldcg(vo + q));
-                vi[o] = diag[q] * (pi[o] * __ldcg(invd + q));
-            }
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                const float v = off[(size_t)j * C + i];
-                const int c = col[(size_t)j * C + i];
-#pragma unroll
-                for (int o = 0; o < 3; ++o) {
-                    const size_t q = 3 * (size_t)c + o;
-                    const float pc = __ldcg(r + q) + bf * (__ldcg(po + q) - of0 * __ldcg(vo + q));
-                    vi[o] += v * (pc * __ldcg(invd + q));
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                pn[q] = pi[o];
-                vn[q] = vi[o];
-                ff_fma(accv[0], r0[q], vi[o]);
-            }
-        }
-        ff r0v[1];
-        cluster_reduce_tree<1>(accv, r0v, sbuf, slots, parity, me, cs);
-        parity ^= 1u;
-        if (threadIdx.x == 0) {
-            const ff d = ff_norm(r0v[0]);
-            if (d.hi == 0.0f) {
-                sc.status = WCFD_KRYLOV_BREAKDOWN;
-                sc.go = 0;
-            } else {
-                sc.alpha = ff_div(sc.rho, d);
-                sc.af = ff_to_float(sc.alpha);
-            }
-        }
-        __syncthreads();
-        if (!sc.go) break;
-        const float af = sc.af;
-        ff acct[2] = {ff_zero(), ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-            float si[3], ti[3];
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                si[o] = __ldcg(r + q) - af * __ldcg(vn + q);
-                x[q] += af * (pn[q] * invd[q]);
-                ti[o] = diag[q] * (si[o] * invd[q]);
-            }
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                const float v = off[(size_t)j * C + i];
-                const int c = col[(size_t)j * C + i];
-#pragma unroll
-                for (int o = 0; o < 3; ++o) {
-                    const size_t q = 3 * (size_t)c + o;
-                    const float scv = __ldcg(r + q) - af * __ldcg(vn + q);
-                    ti[o] += v * (scv * __ldcg(invd + q));
-                }
-            }
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                s[q] = si[o];
-                t[q] = ti[o];
-                ff_fma(acct[0], ti[o], ti[o]);
-                ff_fma(acct[1], ti[o], si[o]);
-            }
-        }
-        ff ts[2];
-        cluster_reduce_tree<2>(acct, ts, sbuf, slots, parity, me, cs);
-        parity ^= 1u;
-        if (threadIdx.x == 0) {
-            const ff tt = ff_norm(ts[0]);
-            sc.omega = tt.hi != 0.0f ? ff_div(ts[1], tt) : ff_zero();
-            sc.of = ff_to_float(sc.omega);
-        }
-        __syncthreads();
-        const float of = sc.of;
-        ff accr[2] = {ff_zero(), ff_zero()};
-        for (int i = i0; i < C; i += stride) {
-#pragma unroll
-            for (int o = 0; o < 3; ++o) {
-                const size_t q = 3 * (size_t)i + o;
-                const float si = s[q];
-                x[q] += of * (si * invd[q]);
-                const float ri = si - of * t[q];
-                r[q] = ri;
-                ff_fma(accr[0], ri, ri);
-                ff_fma(accr[1], r0[q], ri);
-            }
-        }
-        ff rr2[2];
-        cluster_reduce_tree<2>(accr, rr2, sbuf, slots, parity, me, cs);
-        parity ^= 1u;
-        if (threadIdx.x == 0) {
-            sc.rr = ff_norm(rr2[0]);
-            sc.k += 1;
-            if (sc.omega.hi == 0.0f || sc.rho.hi == 0.0f) {
-                sc.status = WCFD_KRYLOV_BREAKDOWN;
-                sc.go = 0;
-            } else {
-                const ff rho_n = ff_norm(rr2[1]);
-                sc.bf = ff_to_float(ff_mul(ff_div(rho_n, sc.rho), ff_div(sc.alpha, sc.omega)));
-                sc.rho = rho_n;
-                sc.go = (sc.k < maxiter && ff_gt(sc.rr, sc.thr2));
-            }
-        }
-        __syncthreads();
-        cur ^= 1;
-    }
-    if (me == 0 && threadIdx.x == 0) {
-        int st = sc.status;
-        if (st == WCFD_OK && !ff_le(sc.rr, sc.thr2)) st = WCFD_NOT_CONVERGED;
-        cse.stats[0].iterations = sc.k;
-        cse.stats[0].status = st;
-        cse.stats[0].residual = sqrt(ff_to_double(sc.rr));
+    if constexpr (SMEM) {
+        BiShared<T> net(records, cap, R);
+        run(net, reinterpret_cast<float*>(records + 3 * (size_t)cap));
+    } else {
+        BiGlobal<T, true> net(ws, sys.C, row0);
+        run(net, nullptr);
     }
 }
 
 template <int W>
-__global__ void __launch_bounds__(CBS) bicgstab_cluster_batched(const wcfd_case* __restrict__ cases, int cs_req) {
-    bicgstab_cluster_body<W>(cases[blockIdx.x / cs_req]);
+__global__ void __launch_bounds__(kBiClusterBlock, 1) bicgstab_cluster_kernel(KrylovArgs a, int R) {
+    const BiSystem sys{a.A.diag, a.A.off, a.A.rhs, a.m.ell_col, nullptr, a.x, a.m.n_cells, a.maxiter, slot_bits(a.m) != 0u, a.atol2, a.rtol2,
+                       a.stats};
+    bicgstab_cluster_body<W, true>(sys, nullptr, R, R);
 }
 
-#define WCFD_W_SWITCH(NAME)                      \
-    switch (W) {                                 \
-        case 0: return (const void*)NAME<0>;     \
-        case 1: return (const void*)NAME<1>;     \
-        case 2: return (const void*)NAME<2>;     \
-        case 3: return (const void*)NAME<3>;     \
-        case 4: return (const void*)NAME<4>;     \
-        case 5: return (const void*)NAME<5>;     \
-        case 6: return (const void*)NAME<6>;     \
-        default: return nullptr;                 \
-    }
+// the momentum system of every case of a table, one cluster a case; cap: the most rows per CTA
+template <int W, bool SMEM>
+__global__ void __launch_bounds__(kBiClusterBlock, 1) bicgstab_cluster_batched(const wcfd_case* __restrict__ cases, int cs_req,
+                                                                              int cap) {
+    const wcfd_case& c = cases[blockIdx.x / cs_req];
+    const BiSystem sys{c.mom.diag, c.mom.off, c.mom.rhs, c.mesh.ell_col, c.mesh.ell_dcol, c.hbya, c.mesh.n_cells, c.prm.maxiter, false,
+                       c.prm.atol_u * c.prm.atol_u, c.prm.rtol_u * c.prm.rtol_u, c.stats + 0};
+    bicgstab_cluster_body<W, SMEM>(sys, c.ws_u.vec, (c.mesh.n_cells + cs_req - 1) / cs_req, cap);
+}
+
+// dynamic shared memory of a CTA of R rows with everything in it, and the most rows that fit
+size_t cluster_bicg_smem_bytes(int R, int W) { return (size_t)R * (48 + 4 * (size_t)(kBiPlanes + 3 * W)); }
+int cluster_bicg_max_rows(int W, int optin) { return (int)(((size_t)optin - 10240) / cluster_bicg_smem_bytes(1, W)); }
 
 // the kernel for R rows a CTA
 template <int W>
@@ -530,6 +348,26 @@ static const void* cg_cluster_pick(int W, int R, bool batched) {
 }
 const void* cg_cluster_kernel_for(int W, int R) { return cg_cluster_pick(W, R, false); }
 const void* cg_cluster_batched_for(int W, int R) { return cg_cluster_pick(W, R, true); }
-const void* bicgstab_cluster_batched_for(int W) { WCFD_W_SWITCH(bicgstab_cluster_batched) }
+const void* bicgstab_cluster_kernel_for(int W) {
+    switch (W) {
+        case 0: return (const void*)bicgstab_cluster_kernel<0>;
+        case 1: return (const void*)bicgstab_cluster_kernel<1>;
+        case 2: return (const void*)bicgstab_cluster_kernel<2>;
+        case 3: return (const void*)bicgstab_cluster_kernel<3>;
+        case 4: return (const void*)bicgstab_cluster_kernel<4>;
+        case 5: return (const void*)bicgstab_cluster_kernel<5>;
+        case 6: return (const void*)bicgstab_cluster_kernel<6>;
+        default: return nullptr;
+    }
+}
+const void* bicgstab_cluster_batched_for(int W, bool resident) {
+#define WCFD_BI(w) \
+    case w: return resident ? (const void*)bicgstab_cluster_batched<w, true> : (const void*)bicgstab_cluster_batched<w, false>;
+    switch (W) {
+        WCFD_BI(0) WCFD_BI(1) WCFD_BI(2) WCFD_BI(3) WCFD_BI(4) WCFD_BI(5) WCFD_BI(6)
+        default: return nullptr;
+    }
+#undef WCFD_BI
+}
 
 }  // namespace wcfd
