@@ -50,6 +50,22 @@ struct BiScalars {
 // (and the neighbours' 1/d_2 where that is not gathered)
 constexpr int kBiPlanes = 24;
 
+// sums of a cluster to thread 0, fin(sums) there; a wait that gave up ends the solve
+template <int NV, int T, bool FENCE, class Fin>
+__device__ __forceinline__ bool cluster_scalars(ff (&acc)[NV], ClusterMeet& meet, BiScalars& sc, Fin&& fin) {
+    const bool met = cluster_reduce<NV, T, false, FENCE>(acc, meet);
+    if (threadIdx.x == 0) {
+        if (met) {
+            fin(acc);
+        } else {
+            sc.status = WCFD_BARRIER_TIMEOUT;
+            sc.go = 0;
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
 // records in the workspace: 13 floats a row (R, U, V, 1/d_2), then the planes r0, p, t; 22 of 27
 // floats.  CLUSTER: the CTAs of a cluster meet, else those of the grid; other CTAs' records are
 // read through L2 in a cluster, whose barrier does not order the first-level caches of two SMs.
@@ -60,10 +76,10 @@ struct BiGlobal {
     float4 *R, *U, *V;
     float *Z, *planes;
     int row0;
-    GridCtl g;
-    ff *sbuf, *slots, *res;
-    uint32_t remote;
-    unsigned phase, me, cs;
+    GridCtl g;          // the grid's
+    ff* sbuf;
+    unsigned phase;
+    ClusterMeet meet;   // the cluster's
     __device__ __forceinline__ BiGlobal(float* ws, int C, int first) : row0(first), phase(0) {
         R = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(ws) + 15) & ~(uintptr_t)15);
         U = R + C;
@@ -87,17 +103,16 @@ struct BiGlobal {
     __device__ __forceinline__ void put_u(int l, float4 w) { U[row0 + l] = w; }
     __device__ __forceinline__ void put_v(int l, float4 w) { V[row0 + l] = w; }
     __device__ __forceinline__ void put_z(int l, float w) { Z[row0 + l] = w; }
+    __device__ __forceinline__ void begin() const {
+        if constexpr (CLUSTER) cluster_begin(meet);
+    }
     // fin(sums) in thread 0, its writes visible to the block; false when a wait gave up
     template <int NV, class Fin>
-    __device__ __forceinline__ bool reduce(ff (&acc)[NV], Fin&& fin) {
-        ++phase;
+    __device__ __forceinline__ bool reduce(ff (&acc)[NV], BiScalars& sc, Fin&& fin) {
         if constexpr (CLUSTER) {
-            cluster_reduce_all<NV, T>(acc, sbuf, slots, res, remote, phase & 1u, me, cs);
-            if (threadIdx.x == 0) fin(acc);
-            __syncthreads();
-            return true;
+            return cluster_scalars<NV, T, true>(acc, meet, sc, fin);
         } else {
-            return grid_reduce<NV, T>(g, acc, sbuf, phase, [&](const ff* s) {
+            return grid_reduce<NV, T>(g, acc, sbuf, ++phase, [&](const ff* s) {
                 if (threadIdx.x == 0) fin(s);
             });
         }
@@ -111,12 +126,10 @@ struct BiShared {
     using Handle = uint32_t;
     static constexpr bool kOwnZ = true;
     float4* R;  // [3][cap]: R, U, V
-    uint32_t base, us, vs;
+    uint32_t us, vs;
     int rows;
-    ff *sbuf, *slots, *res;
-    uint32_t remote;
-    unsigned phase, me, cs;
-    __device__ __forceinline__ BiShared(float4* records, int cap, int rows_per_cta) : R(records), rows(rows_per_cta), phase(0) {
+    ClusterMeet meet;
+    __device__ __forceinline__ BiShared(float4* records, int cap, int rows_per_cta) : R(records), rows(rows_per_cta) {
         us = 16u * cap;
         vs = 32u * cap;
     }
@@ -131,13 +144,10 @@ struct BiShared {
     __device__ __forceinline__ void put_u(int l, float4 w) { R[us / 16 + l] = w; }
     __device__ __forceinline__ void put_v(int l, float4 w) { R[vs / 16 + l] = w; }
     __device__ __forceinline__ void put_z(int, float) {}
+    __device__ __forceinline__ void begin() const { cluster_begin(meet); }
     template <int NV, class Fin>
-    __device__ __forceinline__ bool reduce(ff (&acc)[NV], Fin&& fin) {
-        ++phase;
-        cluster_reduce_all<NV, T>(acc, sbuf, slots, res, remote, phase & 1u, me, cs);
-        if (threadIdx.x == 0) fin(acc);
-        __syncthreads();
-        return true;
+    __device__ __forceinline__ bool reduce(ff (&acc)[NV], BiScalars& sc, Fin&& fin) {
+        return cluster_scalars<NV, T, false>(acc, meet, sc, fin);
     }
 };
 
@@ -233,7 +243,8 @@ __device__ __forceinline__ bool bicgstab_body(const BiSystem& a, Net& net, BiSca
         net.put_u(l, make_float4(ri[0], ri[1], ri[2], di[1]));
         net.put_z(l, di[2]);
     }
-    if (!net.template reduce<2>(acc, [&](const ff* v) {
+    net.begin();
+    if (!net.template reduce<2>(acc, sc, [&](const ff* v) {
             const double rr0 = ff_to_double(v[0]);
             sc.rr = sc.rho = v[0];
             sc.thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * rr0)));
@@ -300,7 +311,7 @@ __device__ __forceinline__ bool bicgstab_body(const BiSystem& a, Net& net, BiSca
             }
             net.put_v(l, make_float4(vi[0], vi[1], vi[2], di[1]));
         }
-        if (!net.template reduce<1>(accv, [&](const ff* r0v) {
+        if (!net.template reduce<1>(accv, sc, [&](const ff* r0v) {
                 if (r0v[0].hi == 0.0f) {
                     sc.status = WCFD_KRYLOV_BREAKDOWN;
                     sc.go = 0;
@@ -356,11 +367,12 @@ __device__ __forceinline__ bool bicgstab_body(const BiSystem& a, Net& net, BiSca
                 else net.planes[(size_t)(6 + o) * C + row0 + l] = ti[o];
             }
         }
-        if (!net.template reduce<2>(acct, [&](const ff* ts) {
+        if (!net.template reduce<2>(acct, sc, [&](const ff* ts) {
                 sc.omega = ts[0].hi != 0.0f ? ff_div(ts[1], ts[0]) : ff_zero();
                 sc.of = ff_to_float(sc.omega);
             }))
             return false;
+        if (!sc.go) break;  // only a wait that gave up
         const float of = sc.of;
         ff accr[2] = {ff_zero(), ff_zero()};
         for (int l = t; l < nloc; l += T) {
@@ -409,7 +421,7 @@ __device__ __forceinline__ bool bicgstab_body(const BiSystem& a, Net& net, BiSca
             net.put_r(l, make_float4(ro[0], ro[1], ro[2], di[0]));
             net.put_u(l, make_float4(uo[0], uo[1], uo[2], di[1]));
         }
-        if (!net.template reduce<2>(accr, [&](const ff* rr2) {
+        if (!net.template reduce<2>(accr, sc, [&](const ff* rr2) {
                 sc.rr = rr2[0];
                 sc.k += 1;
                 if (sc.omega.hi == 0.0f || sc.rho.hi == 0.0f) {

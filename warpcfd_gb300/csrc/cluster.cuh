@@ -22,14 +22,13 @@ __device__ __forceinline__ unsigned cluster_nranks() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The cluster barrier of a reduction: the first n warps (which made the remote slot stores)
-// arrive with release semantics, the other warps arrive relaxed, every thread waits with
-// acquire.  Everything the other warps wrote before the CTA's last __syncthreads happens
-// before warp 0's release (the CTA barrier orders it, and the release is cumulative), so the
-// other CTAs see it after their wait; a release by few threads instead of all.
-template <int N>
-__device__ __forceinline__ void cluster_sync_release() {
-    if (threadIdx.x < 32 * N)
+// The cluster barrier of a reduction: warp 0 (which made the remote slot stores) arrives
+// with release semantics, the other warps arrive relaxed, every thread waits with acquire.
+// Everything the other warps wrote before the CTA's last __syncthreads happens before
+// warp 0's release (the CTA barrier orders it, and the release is cumulative), so the
+// other CTAs see it after their wait; a release by 32 instead of 1,024 threads.
+__device__ __forceinline__ void cluster_sync_warp0_release() {
+    if (threadIdx.x < 32)
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     else
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -105,7 +104,7 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
             if ((unsigned)t < cs) st_cluster_v2f32(map_rank(slots + (parity * NV + i) * 16 + me, t), x.hi, x.lo);
         }
     }
-    cluster_sync_release<1>();
+    cluster_sync_warp0_release();
     if (t < 32) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
@@ -115,6 +114,82 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
             if (t == 0) out[i] = y;
         }
     }
+}
+
+// ---- meetings of a cluster by messages
+// A CTA tells another by an asynchronous remote store that completes bytes on the receiver's
+// mbarrier, so that a reduction costs one trip of its value; the cluster's hardware barrier after
+// remote stores costs their acknowledgement, the arrival and the release: 600 to 1,000 cycles
+// more on 8 to 16 CTAs (per iteration of the CG, two reductions: 16 CTAs 2.71 -> 2.35 us, 8 CTAs
+// 1.62 -> 1.49, 2 CTAs 1.49 -> 1.40).  What the barrier ordered follows from the values: a CTA's total leaves
+// after a block barrier behind all its reads and writes of the pass, and a CTA goes on when it has
+// every CTA's.  A cluster of one CTA needs block barriers only.  Waits are bounded.
+constexpr int kClusterSums = 3;
+template <int T, int SUMS>
+struct ClusterShared {
+    ff slots[2 * kClusterSums * 16];  // [parity][sum][CTA]
+    ff sbuf[SUMS * T];
+    ff res[kClusterSums];
+    unsigned long long bar[2];  // by parity
+    int fail;
+};
+struct ClusterMeet {
+    ff *slots, *sbuf, *res;
+    uint32_t bar, peer_slots, peer_bar;  // own mbarriers; slots and mbarriers of CTA `lane`
+    volatile int* fail;
+    unsigned n, me, cs, width;           // reductions so far; width: 2^k >= cs
+};
+
+__device__ __forceinline__ bool mbarrier_wait(uint32_t bar, unsigned parity) {
+    unsigned spins = 0;
+    uint64_t t0 = 0;
+    for (;;) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((++spins & 1023u) == 0u) {
+            const uint64_t t = global_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > kBarrierTimeoutNs) return false;
+        }
+    }
+}
+// every thread; cluster_begin between this and the first reduction, cluster_end before leaving (no CTA
+// leaves while its shared memory may be addressed)
+template <int T, int SUMS>
+__device__ __forceinline__ ClusterMeet cluster_meet(ClusterShared<T, SUMS>& s) {
+    ClusterMeet m;
+    m.slots = s.slots;
+    m.sbuf = s.sbuf;
+    m.res = s.res;
+    m.fail = &s.fail;
+    m.bar = (uint32_t)__cvta_generic_to_shared(s.bar);
+    m.n = 0;
+    m.me = cluster_rank();
+    m.cs = cluster_nranks();
+    m.width = 1;
+    while (m.width < m.cs) m.width *= 2;
+    const unsigned peer = min((unsigned)(threadIdx.x & 31), m.cs - 1);
+    m.peer_slots = map_rank(s.slots, peer);
+    m.peer_bar = map_rank(s.bar, peer);
+    if (threadIdx.x == 0) {
+        s.fail = 0;
+        for (int i = 0; i < 2; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(m.bar + 8 * i), "r"(1u) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    return m;
+}
+__device__ __forceinline__ void cluster_begin(const ClusterMeet& m) {
+    if (m.cs > 1) cluster_sync_all();
+}
+__device__ __forceinline__ void cluster_end(const ClusterMeet& m) {
+    if (m.cs > 1) cluster_sync_all();
 }
 
 // Row of thread t's u-th in a CTA of T = 256 or 512 threads, and the number of accumulators it
@@ -142,60 +217,82 @@ __device__ __forceinline__ ff cluster_merge(ff (&acc)[kClusterAcc<T>]) {
 }
 
 // Sum NV float-float values (cluster_merge of each thread's accumulators) over the CTAs of the
-// cluster, the sums (normalised, the same bits) in every thread.  Warp i merges value i over
-// the CTA's threads (eight or sixteen per lane, pairwise, then by butterfly) and stores the
-// total into a slot of every CTA (DSMEM); the cluster barrier follows.  With eight warps every
-// warp then merges the cs <= 16 slots, so that no block barrier and no broadcast follows (the
-// eight warps form the scalars redundantly); with sixteen, warp i merges value i and a block
-// barrier passes the sums on.  (Every warp storing its own total to every CTA, eight times the
-// remote stores: 2,000-2,400 cycles a reduction on 16 CTAs against 1,900.)
-// sbuf: [kClusterSums][T]; slots: [2][kClusterSums][16], double-buffered by `parity`; remote:
-// the address of slots in CTA `lane`; res: [kClusterSums] (T = 512).
-constexpr int kClusterSums = 3;
-template <int NV, int T>
-__device__ __forceinline__ void cluster_reduce_all(ff (&v)[NV], ff* sbuf, const ff* slots, ff* res, uint32_t remote,
-                                                   unsigned parity, unsigned me, unsigned cs) {
+// cluster, the sums normalised, the same bits in every CTA: in every thread (ALL), else in warp
+// 0 only.  Warp i merges value i over the CTA's threads (eight or sixteen per lane, pairwise,
+// then by butterfly) and sends the total to every CTA; every warp of a small CTA (ALL, T = 256),
+// warp i (ALL, T = 512) or warp 0 then merges the cs <= 16 totals.  FENCE: global memory
+// written before is visible to the cluster after.  A wait that gives up makes the result false in
+// its thread (not ALL: thread 0, which owns the scalars), or marks m.fail, which a reduction with
+// CHECK turns into false for the whole CTA.
+template <int NV, int T, bool ALL, bool FENCE, bool CHECK = false>
+__device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
     static_assert(NV <= kClusterSums, "three sums at most");
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    const unsigned base = parity * (kClusterSums * 16);
+    const unsigned base = (m.n & 1u) * (kClusterSums * 16);
+    const uint32_t bar = 8u * (m.n & 1u);
+    const unsigned phase = (m.n >> 1) & 1u;
+    ++m.n;
+    const bool alone = m.cs == 1;
+    if (t == 0 && !alone)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(m.bar + bar),
+                     "r"(m.cs * NV * (unsigned)sizeof(ff))
+                     : "memory");
 #pragma unroll
-    for (int i = 0; i < NV; ++i) sbuf[i * T + t] = v[i];
+    for (int i = 0; i < NV; ++i) m.sbuf[i * T + t] = v[i];
     __syncthreads();
+    int failed = 0;
+    if constexpr (CHECK) failed = *m.fail;  // behind the barrier: the same in every thread
     if (wid < NV) {
         ff y[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) y[k] = sbuf[wid * T + 32 * k + lane];
+        for (int k = 0; k < 8; ++k) y[k] = m.sbuf[wid * T + 32 * k + lane];
         if constexpr (T == 512) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) ff_merge(y[k], sbuf[wid * T + 256 + 32 * k + lane]);
+            for (int k = 0; k < 8; ++k) ff_merge(y[k], m.sbuf[wid * T + 256 + 32 * k + lane]);
         }
         ff_tree(y);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(y[0], o);
-        if ((unsigned)lane < cs)
-            st_cluster_v2f32(remote + (base + wid * 16 + me) * (unsigned)sizeof(ff), y[0].hi, y[0].lo);
+        if (alone) {
+            if (lane == 0) m.slots[base + wid * 16] = y[0];
+        } else if ((unsigned)lane < m.cs) {
+            if constexpr (FENCE) __threadfence();
+            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(
+                             m.peer_slots + (base + wid * 16 + m.me) * (unsigned)sizeof(ff)),
+                         "f"(y[0].hi), "f"(y[0].lo), "r"(m.peer_bar + bar)
+                         : "memory");
+        }
     }
-    cluster_sync_release<NV>();
-    if constexpr (T == 256) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) v[i] = (unsigned)(lane & 15) < cs ? slots[base + i * 16 + (lane & 15)] : ff_zero();
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) ff_shfl_merge(v[i], o);
-    } else {
+    const unsigned q = lane & (m.width - 1);
+    if (alone) __syncthreads();
+    if constexpr (ALL && T == 512) {
         if (wid < NV) {
-            ff y = (unsigned)(lane & 15) < cs ? slots[base + wid * 16 + (lane & 15)] : ff_zero();
+            if (!alone && !mbarrier_wait(m.bar + bar, phase)) *m.fail = 1;
+            ff y = q < m.cs ? m.slots[base + wid * 16 + q] : ff_zero();
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) ff_shfl_merge(y, o);
-            if (lane == 0) res[wid] = y;
+            for (int o = 8; o > 0; o >>= 1)
+                if ((unsigned)o < m.width) ff_shfl_merge(y, o);
+            if (lane == 0) m.res[wid] = y;
         }
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < NV; ++i) v[i] = res[i];
+        for (int i = 0; i < NV; ++i) v[i] = m.res[i];
+    } else if (ALL || wid == 0) {
+        if (!alone && !mbarrier_wait(m.bar + bar, phase)) {
+            if constexpr (ALL) *m.fail = 1;
+            else failed = 1;
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = q < m.cs ? m.slots[base + i * 16 + q] : ff_zero();
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+            if ((unsigned)o < m.width)  // the same in every CTA; merging nothing changes nothing
+#pragma unroll
+                for (int i = 0; i < NV; ++i) ff_shfl_merge(v[i], o);
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = ff_norm(v[i]);
+    return failed == 0;
 }
 
 __device__ __forceinline__ float ld_shared_f32(uint32_t addr) {

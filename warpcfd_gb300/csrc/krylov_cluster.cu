@@ -9,17 +9,16 @@
 //  * A neighbour value owned by another CTA is read through distributed shared memory
 //    (mapa + ld.shared::cluster); nothing touches global memory between the set-up and
 //    the final write of x.
-//  * Grid-wide synchronisation is the hardware cluster barrier
-//    (barrier.cluster.arrive.release / wait.acquire), inside the reductions (cluster.cuh): exact
-//    products in float-float (common.cuh), merged in a fixed order, so all CTAs (and all runs)
-//    agree bit for bit.  All CTAs take the same branch at every test, so no CTA can leave
-//    while another still waits or reads its memory.
+//  * The CTAs meet in the reductions only (cluster.cuh): exact products in float-float
+//    (common.cuh), merged in a fixed order, each CTA's total sent to every CTA by a store that
+//    completes bytes on the receiver's mbarrier; so all CTAs (and all runs) agree bit for bit and
+//    take the same branch at every test.
 //  * The direction update p = z + beta p is evaluated inside the SpMV for the row and its
-//    neighbours, so an iteration needs two barriers.
+//    neighbours, so an iteration needs two reductions.
 // Bound by the latency of its two reductions and, with many rows a CTA, by instruction issue.
-// Measured per iteration (1,024 threads with everything in shared memory -> this form): 2 CTAs
-// x 512 rows 2.76 -> 1.57 us, 8 x 512 2.88 -> 1.64, 16 x 2,000 3.77 -> 2.7, 16 x 4,096 4.69 ->
-// 3.74 (the grid kernel: 4.59).
+// Measured per iteration (1,024 threads, everything in shared memory, cluster barriers -> this
+// form): 2 CTAs x 512 rows 2.71 -> 1.40 us, 8 x 512 2.87 -> 1.49, 16 x 2,000 3.77 -> 2.35, 16 x 4,096
+// 4.69 -> 3.45 (the grid kernel: 4.59).
 // The arithmetic is that of cg_kernel (krylov.cu): the same Jacobi-preconditioned CG with
 // fp64-accurate dot products and the same stop test.
 #include "bicgstab.cuh"
@@ -52,14 +51,13 @@ int cluster_cg_max_rows(int W, int optin) {
 template <int W, int RPT, int T>
 __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ ff slots[2 * kClusterSums * 16], sbuf[kClusterSums * T], res[kClusterSums];
+    __shared__ __align__(16) ClusterShared<T, 3> meeting;
     constexpr int WA = W > 0 ? W : 1, NA = kClusterAcc<T>;
     constexpr int GR = T == 512 ? 2 : RPT < 4 ? RPT : 4;  // rows whose gathers are in flight together
     constexpr bool REG = T == 256;                        // the matrix in registers
     constexpr int RM = REG ? RPT : 1;
     const int C = a.m.n_cells;
     const unsigned me = cluster_rank();
-    const unsigned cs = cluster_nranks();
     const int row0 = (int)me * R;
     const int nloc = max(0, min(R, C - row0));
     float2* zp = reinterpret_cast<float2*>(smem);         // [RPT T] (z, p), by row
@@ -68,7 +66,7 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
     float* s_i = s_d + RPT * T;                           // [RPT][T]
     const int t = threadIdx.x;
     const int groups = (nloc + GR * T - 1) / (GR * T);  // groups of GR rows a thread that hold any
-    const uint32_t remote = map_rank(slots, min((unsigned)(t & 31), cs - 1));
+    ClusterMeet meet = cluster_meet(meeting);
     const uint32_t zp0 = (uint32_t)__cvta_generic_to_shared(zp);
 
     // the matrix rows of this thread; at: where a neighbour's pair lies, here or in another CTA
@@ -131,10 +129,9 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
         }
         if (__all_sync(0xffffffffu, mine)) local |= 1u << u;
     }
-    unsigned parity = 0;
     ff acc[3] = {cluster_merge<T>(arr), cluster_merge<T>(arz), cluster_merge<T>(abb)};
-    cluster_reduce_all<3, T>(acc, sbuf, slots, res, remote, parity, me, cs);
-    parity ^= 1u;
+    cluster_begin(meet);
+    cluster_reduce<3, T, true, false>(acc, meet);
     ff rr = acc[0], rz = acc[1];
     const ff thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * ff_to_double(rr))));
     if (me == 0 && t == 0) {
@@ -195,8 +192,10 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
         }
         ff accq[1] = {cluster_merge<T>(apq)};
-        cluster_reduce_all<1, T>(accq, sbuf, slots, res, remote, parity, me, cs);
-        parity ^= 1u;
+        if (!cluster_reduce<1, T, true, false, true>(accq, meet)) {
+            status = WCFD_BARRIER_TIMEOUT;
+            break;
+        }
         if (accq[0].hi == 0.0f) {
             status = WCFD_KRYLOV_BREAKDOWN;
             break;
@@ -223,8 +222,7 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
         }
         ff acc2[2] = {cluster_merge<T>(arr), cluster_merge<T>(arz)};
-        cluster_reduce_all<2, T>(acc2, sbuf, slots, res, remote, parity, me, cs);
-        parity ^= 1u;
+        cluster_reduce<2, T, true, false>(acc2, meet);
         rr = acc2[0];
         bf = rz.hi != 0.0f ? ff_div_to_float(acc2[1], rz) : 0.0f;
         rz = acc2[1];
@@ -235,7 +233,9 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
         const int l = cluster_row<T>(t, u);
         if (l < nloc) a.x[row0 + l] = xr[u];
     }
+    cluster_end(meet);
     if (me == 0 && t == 0) {
+        if (*meet.fail) status = WCFD_BARRIER_TIMEOUT;
         if (status == WCFD_OK && !ff_le(rr, thr2)) status = WCFD_NOT_CONVERGED;
         a.stats->iterations = k;
         a.stats->status = status;
@@ -279,18 +279,14 @@ __device__ __forceinline__ void bicgstab_cluster_body(const BiSystem& sys, float
     constexpr int T = kBiClusterBlock;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ BiScalars sc;
-    __shared__ ff slots[2 * kClusterSums * 16], sbuf[2 * T], res[kClusterSums];
-    const unsigned me = cluster_rank(), cs = cluster_nranks();
+    __shared__ __align__(16) ClusterShared<T, 2> meeting;
+    const unsigned me = cluster_rank();
     const int row0 = (int)me * R, nloc = max(0, min(R, sys.C - row0));
     float4* records = reinterpret_cast<float4*>(smem);
     auto run = [&](auto& net, float* own) {
-        net.sbuf = sbuf;
-        net.slots = slots;
-        net.res = res;
-        net.me = me;
-        net.cs = cs;
-        net.remote = map_rank(slots, min((unsigned)(threadIdx.x & 31), cs - 1));
+        net.meet = cluster_meet(meeting);
         bicgstab_body<W, T, SMEM>(sys, net, sc, own, cap, row0, nloc, me == 0);
+        cluster_end(net.meet);
     };
     if constexpr (SMEM) {
         BiShared<T> net(records, cap, R);

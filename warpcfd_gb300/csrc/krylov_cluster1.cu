@@ -267,56 +267,10 @@ size_t cluster_cg1m_smem_bytes(int R, int W) {
     return 4 * (size_t)cap + (cap > 2048 ? (4 * (size_t)W + 8) * cap : 0);
 }
 
-// Sum three float-float values over the cluster's CTAs, the sums (normalised, the same bits) to
-// thread 0.  acc[i][q]: the accumulators of value i.  Warp i merges value i over the CTA's
-// threads and stores it to every CTA's slots; a cluster of one CTA needs neither DSMEM nor
-// the cluster barrier.  sbuf: [3][T]; slots: [2][3][16], double-buffered by `parity`.
-template <int T>
-__device__ __forceinline__ void cg1m_reduce(ff (&acc)[3][kClusterAcc<T>], ff (&out)[3], ff* sbuf, ff* slots, unsigned parity,
-                                            unsigned me, unsigned cs) {
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    const unsigned base = parity * 48;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        ff_merge(acc[i][0], acc[i][1]);
-        if constexpr (T == 256) {
-            ff_merge(acc[i][2], acc[i][3]);
-            ff_merge(acc[i][0], acc[i][2]);
-        }
-        sbuf[i * T + t] = acc[i][0];
-    }
-    __syncthreads();
-    if (wid < 3) {
-        ff y[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) y[k] = sbuf[wid * T + 32 * k + lane];
-        if constexpr (T == 512) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) ff_merge(y[k], sbuf[wid * T + 256 + 32 * k + lane]);
-        }
-        ff_tree(y);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ff_shfl_merge(y[0], o);
-        if ((unsigned)lane < cs) st_cluster_v2f32(map_rank(slots + base + wid * 16 + me, lane), y[0].hi, y[0].lo);
-    }
-    if (cs > 1) cluster_sync_release<3>();
-    else __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) out[i] = (unsigned)lane < cs ? slots[base + i * 16 + lane] : ff_zero();
-        if (cs > 1) {
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1)  // lanes 0..15 hold the cs <= 16 slots
-#pragma unroll
-                for (int i = 0; i < 3; ++i) ff_shfl_merge(out[i], o);
-        }
-    }
-}
-
 template <int W, int RPT, int T>
 __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ ff slots[2 * 3 * 16], sbuf[3 * T];
+    __shared__ __align__(16) ClusterShared<T, 3> meeting;
     struct Scal {
         ff rr, gamma, thr2;
         float af, bf, alpha_prev;
@@ -328,7 +282,6 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
     constexpr int RM = REG ? RPT : 1;
     const int C = a.m.n_cells;
     const unsigned me = cluster_rank();
-    const unsigned cs = cluster_nranks();
     const int row0 = (int)me * R;
     const int nloc = max(0, min(R, C - row0));
     float* ub = reinterpret_cast<float*>(smem);   // [RPT T] u = M r, by row
@@ -337,6 +290,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
     float* s_i = s_d + RPT * T;                   // [RPT][T]
     const int t0 = threadIdx.x;
     const int groups = (nloc + GR * T - 1) / (GR * T);  // groups of GR rows a thread that hold any
+    ClusterMeet meet = cluster_meet(meeting);
     const uint32_t ub0 = (uint32_t)__cvta_generic_to_shared(ub);
 
     // this thread's rows of the matrix; at: where a neighbour's u lies, here or in another CTA
@@ -400,10 +354,9 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         }
         if (__all_sync(0xffffffffu, mine)) local |= 1u << u;
     }
-    unsigned parity = 0;
-    ff red[3];
-    cg1m_reduce<T>(acc, red, sbuf, slots, parity, me, cs);
-    parity ^= 1u;
+    ff red[3] = {cluster_merge<T>(acc[0]), cluster_merge<T>(acc[1]), cluster_merge<T>(acc[2])};
+    cluster_begin(meet);
+    const bool met0 = cluster_reduce<3, T, false, false>(red, meet);
     if (t0 == 0) {
         const double rr0 = ff_to_double(red[0]);
         sc.thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * rr0)));
@@ -411,14 +364,14 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         sc.bf = 0.0f;
         sc.alpha_prev = 0.0f;
         sc.k = -1;
-        sc.status = WCFD_OK;
-        sc.go = 1;
+        sc.status = met0 ? WCFD_OK : WCFD_BARRIER_TIMEOUT;
+        sc.go = met0;
         if (me == 0) {
             a.stats->initial_residual = sqrt(rr0);
             a.stats->rhs_norm = sqrt(ff_to_double(red[2]));
         }
     }
-    __syncthreads();  // the barrier above also published u0 to every CTA
+    __syncthreads();  // the reduction also published u0 to every CTA
     while (sc.go) {
         const float af = sc.af, bf = sc.bf;
         // (1) s = w + beta s ; p = u + beta p ; x += alpha p ; r -= alpha s ; u = M r
@@ -439,7 +392,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
                     ub[cluster_row<T>(t0, u)] = ur[u];
                 }
             }
-            if (cs > 1) cluster_sync_all();  // every CTA's new u, visible to the cluster
+            if (meet.cs > 1) cluster_sync_all();  // every CTA's new u, visible to the cluster
             else __syncthreads();
         }
         // (2) w = A u ; r.r ; r.u ; w.u.  The gathers of GR rows are issued before the first is used.
@@ -489,11 +442,13 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
                 ff_fma(acc[2][u % NA], wi, ur[u]);
             }
         }
-        ff d3[3];
-        cg1m_reduce<T>(acc, d3, sbuf, slots, parity, me, cs);
-        parity ^= 1u;
-        if (t0 == 0) {
-            const ff rr = ff_norm(d3[0]), gamma = ff_norm(d3[1]), delta = ff_norm(d3[2]);
+        ff d3[3] = {cluster_merge<T>(acc[0]), cluster_merge<T>(acc[1]), cluster_merge<T>(acc[2])};
+        const bool met = cluster_reduce<3, T, false, false>(d3, meet);
+        if (t0 == 0 && !met) {
+            sc.status = WCFD_BARRIER_TIMEOUT;
+            sc.go = 0;
+        } else if (t0 == 0) {
+            const ff rr = d3[0], gamma = d3[1], delta = d3[2];
             sc.rr = rr;
             sc.k += 1;  // x now holds k updates
             if (!(sc.k < a.maxiter && ff_gt(rr, sc.thr2))) {
@@ -525,6 +480,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         const int l = cluster_row<T>(t0, u);
         if (l < nloc) a.x[row0 + l] = xr[u];
     }
+    cluster_end(meet);
     if (me == 0 && t0 == 0) {
         int st = sc.status;
         if (st == WCFD_OK && !ff_le(sc.rr, sc.thr2)) st = WCFD_NOT_CONVERGED;
