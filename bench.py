@@ -606,7 +606,7 @@ def run_ours(args):
                    "fields_finite": finite,
                    "momentum_rel_residual": {"first": float(rel_res[0]), "last": float(rel_res[-1])}},
         "e2e": e2e,
-        "gpu_launches": (6 + 7 * solver.NUM_INNER_LOOPS) * K_,
+        "gpu_launches": (5 + 7 * solver.NUM_INNER_LOOPS) * K_,
         "roofline": {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peaks
                      else "fallback", "traffic": traffic,

@@ -1,6 +1,7 @@
 // Host side of the batched form: one SIMPLE outer iteration (or PISO step) for every case
 // of a device case table, as a fixed sequence of batched launches (capturable in a CUDA
 // graph: the sequence depends only on the dims, never on the data).
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
@@ -226,10 +227,9 @@ extern "C" int wcfd_batch_simple_iteration(const wcfd_case* cases, int32_t n_cas
     int rc = launch_cluster(bi.fn, n_cases, cs, kBiClusterBlock, bi.smem, st, bargs);
     if (rc) return rc;
     // :118-123
-    hbya_batched<<<gc, fb, 0, st>>>(cases);
-    BCHECK("hbya_batched");
-    rua_faces_batched<<<gf, fb, 0, st>>>(cases);
-    BCHECK("rua_faces_batched");
+    const dim3 gfc((std::max(d.max_faces, d.max_cells) + fb - 1) / fb, n_cases);
+    hbya_rua_faces_batched<<<gfc, fb, 0, st>>>(cases);
+    BCHECK("hbya_rua_faces_batched");
     const size_t smem = batch_cg_smem(d, R);
     for (int inner = 0; inner < d.n_inner; ++inner) {
         for (int ortho = 0; ortho < d.n_ortho; ++ortho) {

@@ -743,7 +743,7 @@ int wcfd_simple_iteration(const wcfd_case* cp, void* stream) {
     // the face kernels are persistent: resident blocks striding over the faces
     const int gfa = resident_grid((const void*)face_pass_kernel, m.n_faces);
     const int gfp = resident_grid((const void*)face_pass_partial_kernel, m.n_faces);
-    const int gfc = resident_grid((const void*)cell_to_face_kernel, m.n_faces);
+    const int gfc = resident_grid((const void*)hbya_rua_faces_kernel, m.n_faces);
     // incompressible.py:96-99
     face_pass_kernel<<<gfa, kBlock, 0, st>>>(m, c.bc, c.state, WCFD_ALL, 1u | 2u | skew | (c.prm.rhie_chow ? 16u : 0u),
                                             c.rua_faces);
@@ -764,10 +764,9 @@ int wcfd_simple_iteration(const wcfd_case* cp, void* stream) {
     if (rc) return rc;
     mark(1);
     // :118-123
-    hbya_kernel<<<gc, kBlock, 0, st>>>(m.n_cells, c.state.cell_gradients, c.rua, c.hbya, c.state.cell_values);
-    LAUNCH_CHECK("hbya_kernel");
-    cell_to_face_kernel<<<gfc, kBlock, 0, st>>>(m, c.rua, c.rua_faces);
-    LAUNCH_CHECK("cell_to_face_kernel");
+    hbya_rua_faces_kernel<<<gc + gfc, kBlock, 0, st>>>(m, gc, c.state.cell_gradients, c.rua, c.hbya, c.state.cell_values,
+                                                       c.rua_faces);
+    LAUNCH_CHECK("hbya_rua_faces_kernel");
     for (int inner = 0; inner < c.prm.n_inner; ++inner) {
         NvtxRange r("wcfd pressure corrector");
         for (int ortho = 0; ortho < c.prm.n_ortho; ++ortho) {

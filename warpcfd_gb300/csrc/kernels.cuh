@@ -19,7 +19,8 @@ __global__ void boundary_values_kernel(wcfd_mesh m, wcfd_bc bc, wcfd_state s);
 __global__ void mass_flux_kernel(wcfd_mesh m, wcfd_state s);
 __global__ void div_kernel(wcfd_mesh m, const float* mdot, float* div);
 __global__ void cell_to_face_kernel(wcfd_mesh m, const float* x, float* y);
-__global__ void hbya_kernel(int C, const float* grad, const float* rua, float* hbya, float* cell_values);
+__global__ void hbya_rua_faces_kernel(wcfd_mesh m, int cell_blocks, const float* grad, const float* rua, float* hbya,
+                                      float* cell_values, float* rua_faces);
 __global__ void p_update_kernel(int C, const float* p_new, float* cell_values, float alpha);
 
 // assembly launches; xt selects the kernels with the opt-in explicit internal terms
@@ -49,8 +50,7 @@ __global__ void add_rhs_kernel(int64_t n, float* rhs, const float* a, float scal
 __global__ void face_pass_batched(const wcfd_case* cases, uint32_t mask, uint32_t flags);
 __global__ void face_pass_partial_batched(const wcfd_case* cases, uint32_t mask, uint32_t flags);
 __global__ void gradient_batched(const wcfd_case* cases, uint32_t mask, int mode);
-__global__ void hbya_batched(const wcfd_case* cases);
-__global__ void rua_faces_batched(const wcfd_case* cases);
+__global__ void hbya_rua_faces_batched(const wcfd_case* cases);
 __global__ void p_update_batched(const wcfd_case* cases);
 void launch_assemble_batched(bool pressure, bool xt, dim3 grid, int block, cudaStream_t st, const wcfd_case* cases);
 
