@@ -54,11 +54,11 @@ METRIC = "cell-iterations/s"
 # (`dram__bytes_read.sum + dram__bytes_write.sum`, one capture per workload):
 #   channel   cg_cluster_kernel: 1.47 MB per launch whatever the iteration count (the
 #             system is read once into shared memory)
-#   cavity3d  cg_kernel (int16 column offsets): 15.40 GB for a 174-iteration launch =
-#             88.5 MB per iteration (the vectors stay in L2; the matrix streams)
+#   cavity3d  cg_kernel (off-diagonals in place): 178 MB for a launch of 100 iterations (the
+#             matrix and the vectors stay in L2 and shared memory; set-up included)
 MEASURED_TRAFFIC = {
     "channel": {"per_launch": 1.473e6, "per_iteration": 0.0},
-    "cavity3d": {"per_launch": 0.0, "per_iteration": 15.403e9 / 174},
+    "cavity3d": {"per_launch": 177.6e6, "per_iteration": 0.0},
 }
 
 
@@ -572,10 +572,13 @@ def run_ours(args):
     from warpcfd_gb300 import _lib
     rows = int(_lib.load().wcfd_batch_max_rows(W))  # rows per CTA of the cluster-resident CG
     grid_cg = C > 16 * rows
-    # the grid CG streams int16 column offsets when the mesh has them (wcfd_mesh.ell_dcol)
-    col_bytes = 2 if grid_cg and g.get("ell_dcol") is not None else 4
+    # the grid kernels stream int16 column offsets when the mesh has them (wcfd_mesh.ell_dcol); the
+    # CG streams no columns where the off-diagonals stand in place (wcfd_mesh.slot_mask)
+    offsets = 2 if grid_cg and g.get("ell_dcol") is not None else 4
+    in_place = grid_cg and (model.mesh_struct().slot_mask & 0xFFFF0000) == _lib.SLOT_MASK
+    col_bytes = 0 if in_place else offsets
     cg_bytes = sum(perfmodel.cg_bytes(C, W, int(k), col_bytes) for k in k_p)
-    bi_bytes = sum(perfmodel.bicgstab_bytes(C, W, int(k)) for k in k_u)
+    bi_bytes = sum(perfmodel.bicgstab_bytes(C, W, int(k), offsets) for k in k_u)
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))

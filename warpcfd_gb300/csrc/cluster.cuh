@@ -1,6 +1,6 @@
 // Thread-block-cluster primitives shared by the cluster-resident solvers: rank queries,
-// the hardware cluster barrier, distributed-shared-memory loads and stores, and a
-// deterministic float-float reduction over the CTAs of a cluster.
+// the hardware cluster barrier, distributed-shared-memory loads and stores, and
+// deterministic float-float reductions over the CTAs of a cluster (by that barrier or by messages).
 #pragma once
 
 #include "common.cuh"

@@ -13,8 +13,8 @@ namespace wcfd {
 
 constexpr int kBlock = 256;      // threads of the one-thread-per-face/cell kernels
 constexpr int kMaxFieldBlock = 512;  // largest block of the batched field kernels (a launch parameter)
-constexpr int kSolverBlock = 1024;  // threads of the persistent Krylov kernels (one block per SM)
-constexpr int kCgBlock = 512;       // threads of the persistent CG (one block per SM)
+constexpr int kSolverBlock = 1024;  // threads of the barrier check, whose residency caps the Krylov grids
+constexpr int kCgBlock = 512;       // threads of the persistent CG and BiCGSTAB (one block per SM)
 constexpr int kMaxSlots = 6;     // faces per cell (hex)
 // face reference of a null slot: a cell of a mixed mesh with fewer faces than the
 // mesh's faces_per_cell (a wedge or a tetrahedron among hexes); its weights are zero

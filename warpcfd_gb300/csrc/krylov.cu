@@ -1,15 +1,14 @@
-// Persistent Krylov solvers: one cooperative launch per solve, rows distributed
-// grid-stride over all co-resident blocks, fp64-accurate dot products (exact products
-// summed in float-float across threads, warps and blocks; common.cuh) reduced deterministically
+// Persistent Krylov solvers: one cooperative launch per solve, contiguous rows per
+// co-resident block, fp64-accurate dot products (exact products summed
+// in float-float across threads, warps and blocks; common.cuh) reduced deterministically
 // at bounded grid barriers.  They replace warp.optim.linear.cg /
 // bicgstab with the diagonal (Jacobi) preconditioner as called by Equation.solve_Axb
 // (warp_cfd/FV/terms/equation.py:195-200).  Stop test: ||r||_2 <= atol before an
 // iteration, or maxiter iterations.
 //
-// Each search-direction update (CG: p = z + beta p; BiCGSTAB: p = r + beta (p - omega v),
-// s = r - alpha v) is evaluated on the fly inside the SpMV that consumes it, for the row
-// itself and for every gathered neighbour, and the new direction is written to the other
-// half of a double buffer.  The arithmetic is the textbook algorithm's, but a CG iteration
+// Each search-direction update (CG: p = z + beta p, p double-buffered; BiCGSTAB, bicgstab.cuh:
+// p = r + beta (p - omega v), s = r - alpha v) is evaluated on the fly inside the SpMV that
+// consumes it, for the row itself and for every gathered neighbour.  The arithmetic is the textbook algorithm's, but a CG iteration
 // needs two grid barriers instead of three and a BiCGSTAB iteration three instead of five.
 //
 // The scalar recurrences (alpha, beta, omega, the stop test) run on the float-float sums

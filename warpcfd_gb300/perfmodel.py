@@ -9,13 +9,13 @@ from __future__ import annotations
 
 
 def cg_bytes_per_iteration(C: int, W: int, col_bytes: int = 4) -> int:
-    """One CG iteration (two passes) per row:
-    p = z + beta p_old ; q = A p ; x += alpha_prev p_old :
-                   off 4W + col (col_bytes) W + diag 4 + z 4 + p_old 4 + x 8 (rw) + p 4 (w) + q 4 (w)
-    r -= alpha q ; z = M r : r 8 (rw) + q 4 + invd 4 + z 4 (w)
-    col_bytes 2 when the columns are read as int16 offsets (wcfd_mesh.ell_dcol).
+    """One CG iteration (two passes) per row, r, q, x and 1/diag held in shared memory:
+    p = z + beta p_old ; q = A p : off 4W + col (col_bytes) W + diag 4 + z 4 + p_old 4 + p 4 (w)
+    r -= alpha q ; z = M r       : z 4 (w)
+    col_bytes 2 when the columns are read as int16 offsets (wcfd_mesh.ell_dcol), 0 when the
+    off-diagonals stand in place (wcfd_mesh.slot_mask) and a chunk of rows shares its offsets.
     """
-    return C * ((4 + col_bytes) * W + 28 + 20)
+    return C * ((4 + col_bytes) * W + 20)
 
 
 def cg_bytes_setup(C: int, W: int, col_bytes: int = 4) -> int:
@@ -27,20 +27,26 @@ def cg_bytes(C: int, W: int, iters: int, col_bytes: int = 4) -> int:
     return cg_bytes_setup(C, W, col_bytes) + iters * cg_bytes_per_iteration(C, W, col_bytes)
 
 
-def bicgstab_bytes_per_iteration(C: int, W: int) -> int:
-    """One BiCGSTAB iteration on the 3-component system, per cell (12 B per vector):
-    v = A M p : off/col 8W + diag 12 + p 12 + invd 12 + v 12 + r0 12
-    s, x      : r 24 + v 12 + x 24 + p 12 + invd 12
-    t = A M s : off/col 8W + diag 12 + s 12 + invd 12 + t 12
-    x, r      : x 24 + s 12 + invd 12 + t 12 + r 12 + r0 12
-    p         : r 12 + p 24 + v 12
+BICG_RESIDENT_ROWS = 152 * 227 * 1024  # over the bytes of a row: what the grid's shared memory holds
+
+
+def bicgstab_bytes_per_iteration(C: int, W: int, col_bytes: int = 4) -> int:
+    """One BiCGSTAB iteration on the 3-component system, per cell; records R = (r, 1/d_0),
+    U = (u, 1/d_1), V = (v, 1/d_1) of 16 B and Z = 1/d_2 of 4 B:
+    v = A M p : R, U, Z 36 + V 16 (w)
+    t = A M s : R, V, Z 36
+    x, r, u   : R, U 32 (w)
+    A resident system moves those; a streamed one also off/col (4 + col_bytes) W + diag 12 in
+    each product, r0 12 + p 12 (w), t 12 (w), and R, V, Z 36 + r0, p, t, x 48 + x 12 (w).
     """
-    return C * (16 * W + 60 + 84 + 48 + 84 + 48)
+    if C * (96 + 8 * W) <= BICG_RESIDENT_ROWS:
+        return C * 120
+    return C * (2 * (4 + col_bytes) * W + 276)
 
 
-def bicgstab_bytes(C: int, W: int, iters: int) -> int:
+def bicgstab_bytes(C: int, W: int, iters: int, col_bytes: int = 4) -> int:
     setup = C * (8 * W + 12 + 12 + 12 + 12 * 4)
-    return setup + iters * bicgstab_bytes_per_iteration(C, W)
+    return setup + iters * bicgstab_bytes_per_iteration(C, W, col_bytes)
 
 
 def face_pass_bytes(C: int, K: int, Ki: int, B: int, mdot: bool = True) -> int:
@@ -82,7 +88,7 @@ def simple_step_bytes(C, K, Ki, B, F, W, k_u, k_p, n_corr=1, col_bytes=4) -> dic
         + gradient_bytes(C, K, F) * n_corr,
         "momentum_assemble": momentum_assembly_bytes(C, K, F, W, B),
         "pressure_assemble": pressure_assembly_bytes(C, K, F, W, B) * n_corr,
-        "bicgstab": bicgstab_bytes(C, W, k_u),
+        "bicgstab": bicgstab_bytes(C, W, k_u, max(col_bytes, 2)),
         "cg": cg_bytes(C, W, k_p, col_bytes) * n_corr,
         "small": 32 * C + 12 * K,
     }
