@@ -166,6 +166,7 @@ _SIGS = {
                                   ct.POINTER(MeshFaces_t), vp]),
     "wcfd_mesh_last_error": (ct.c_char_p, []),
     "wcfd_check_mesh": (ct.c_int, [ct.POINTER(Mesh_t), ct.POINTER(ct.c_int32), vp]),
+    "wcfd_cluster_meeting_check": (ct.c_int, [ct.c_int32] * 6 + [ct.c_int64, ct.c_int64, ct.POINTER(ct.c_int32), vp]),
     "wcfd_grid_barrier_check": (ct.c_int, [ct.c_int32, ct.c_int32, ct.POINTER(ct.c_int32), vp]),
 }
 

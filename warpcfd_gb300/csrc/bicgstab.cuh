@@ -445,7 +445,7 @@ __device__ __forceinline__ bool bicgstab_body(const BiSystem& a, Net& net, BiSca
         if (st == WCFD_OK && !ff_le(sc.rr, sc.thr2)) st = WCFD_NOT_CONVERGED;
         a.stats->iterations = sc.k;
         a.stats->status = st;
-        a.stats->residual = sqrt(ff_to_double(sc.rr));
+        a.stats->residual = st == WCFD_BARRIER_TIMEOUT ? -1.0 : sqrt(ff_to_double(sc.rr));
     }
     return true;
 }

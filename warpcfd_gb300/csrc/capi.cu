@@ -416,6 +416,42 @@ int wcfd_grid_barrier_check(int32_t skip_block, int32_t phases, int32_t* result,
     return rc;
 }
 
+int wcfd_cluster_meeting_check(int32_t ctas, int32_t threads, int32_t every_warp, int32_t reductions, int32_t who, int32_t at,
+                               int64_t delay_ns, int64_t limit_ns, int32_t* result, void* stream) {
+    RET_IF(!result || ctas < 2 || ctas > 16 || (ctas & (ctas - 1)) || (threads != 256 && threads != 512), WCFD_ERR_ARGUMENT,
+           "2 to 16 CTAs (a power of two) of 256 or 512 threads, and a result array");
+    RET_IF(reductions < 1 || reductions > 100000 || who < -1 || who >= ctas || at < 0, WCFD_ERR_ARGUMENT, "bad reductions, who or at");
+    RET_IF(delay_ns > 1000000000 || limit_ns < 1000 || limit_ns > 1500000000, WCFD_ERR_ARGUMENT,
+           "a delay of at most 1 s, a limit of 1 us to 1.5 s");
+    cudaStream_t st = S(stream);
+    const void* fn = cluster_check_kernel_for(threads, every_warp != 0);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int* dev = nullptr;
+    if (cudaMalloc(&dev, 16 * sizeof(int)) != cudaSuccess) return check_launch("cluster check: allocation");
+    long long delay = delay_ns, limit = limit_ns;
+    void* args[] = {&reductions, &who, &at, &delay, &limit, &dev};
+    int rc = WCFD_OK;
+    if (cudaMemsetAsync(dev, 0xff, 16 * sizeof(int), st) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaLaunchKernelExC(&cfg, fn, args) != cudaSuccess ||
+        cudaMemcpyAsync(result, dev, ctas * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
+        rc = check_launch("cluster check");
+        if (rc == WCFD_OK) rc = set_error(WCFD_ERR_CUDA, "cluster check failed");
+    }
+    cudaFree(dev);
+    return rc;
+}
+
 int64_t wcfd_krylov_workspace_floats(int32_t n_cells, int32_t ncomp) {
     if (n_cells <= 0 || (ncomp != 1 && ncomp != 3)) return -1;
     return ncomp == 1 ? 6LL * n_cells : 27LL * n_cells;

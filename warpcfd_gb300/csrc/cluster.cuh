@@ -136,34 +136,44 @@ struct ClusterShared {
 struct ClusterMeet {
     ff *slots, *sbuf, *res;
     uint32_t bar, peer_slots, peer_bar;  // own mbarriers; slots and mbarriers of CTA `lane`
-    volatile int* fail;
+    volatile int* fail;                  // a wait of this CTA gave up (ALL with 512 threads)
     unsigned n, me, cs, width;           // reductions so far; width: 2^k >= cs
+    uint64_t limit;                      // of a wait, ns
 };
 
-__device__ __forceinline__ bool mbarrier_wait(uint32_t bar, unsigned parity) {
-    unsigned spins = 0;
-    uint64_t t0 = 0;
-    for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if ((++spins & 1023u) == 0u) {
-            const uint64_t t = global_ns();
-            if (t0 == 0) t0 = t;
-            if (t - t0 > kBarrierTimeoutNs) return false;
-        }
+__device__ __forceinline__ bool mbarrier_try(uint32_t bar, unsigned parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// Wait for the phase of one of this CTA's mbarriers, `limit` ns at most.  Every thread of the CTA that
+// waits for a phase gets the same answer, whichever gives up first: a thread whose time is up makes the
+// mbarrier expect kGiveUpBytes that nobody sends and looks again.  Either the phase was complete before
+// that, and then every thread sees it (and the next phase of this mbarrier is the one that cannot
+// complete), or it never completes.  So a warp that goes on and a warp that leaves cannot part.
+// The threads of a block add less than the 2^20 - 1 bytes that an mbarrier counts.
+constexpr unsigned kGiveUpBytes = 512;  // more than the totals of a reduction (16 CTAs x 3 sums x 8)
+__device__ __forceinline__ bool mbarrier_wait(uint32_t bar, unsigned parity, uint64_t limit) {
+    if (mbarrier_try(bar, parity)) return true;
+    const uint64_t t0 = global_ns();
+    while (!mbarrier_try(bar, parity)) {
+        if (global_ns() - t0 <= limit) continue;
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(kGiveUpBytes) : "memory");
+        return mbarrier_try(bar, parity);
     }
+    return true;
 }
 // every thread; cluster_begin between this and the first reduction, cluster_end before leaving (no CTA
 // leaves while its shared memory may be addressed)
 template <int T, int SUMS>
-__device__ __forceinline__ ClusterMeet cluster_meet(ClusterShared<T, SUMS>& s) {
+__device__ __forceinline__ ClusterMeet cluster_meet(ClusterShared<T, SUMS>& s, uint64_t limit = kBarrierTimeoutNs) {
     ClusterMeet m;
+    m.limit = limit;
     m.slots = s.slots;
     m.sbuf = s.sbuf;
     m.res = s.res;
@@ -221,10 +231,9 @@ __device__ __forceinline__ ff cluster_merge(ff (&acc)[kClusterAcc<T>]) {
 // 0 only.  Warp i merges value i over the CTA's threads (eight or sixteen per lane, pairwise,
 // then by butterfly) and sends the total to every CTA; every warp of a small CTA (ALL, T = 256),
 // warp i (ALL, T = 512) or warp 0 then merges the cs <= 16 totals.  FENCE: global memory
-// written before is visible to the cluster after.  A wait that gives up makes the result false in
-// its thread (not ALL: thread 0, which owns the scalars), or marks m.fail, which a reduction with
-// CHECK turns into false for the whole CTA.
-template <int NV, int T, bool ALL, bool FENCE, bool CHECK = false>
+// written before is visible to the cluster after.  False when the wait gave up: in every thread of
+// the CTA (ALL), else in thread 0, which owns the scalars.
+template <int NV, int T, bool ALL, bool FENCE>
 __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
     static_assert(NV <= kClusterSums, "three sums at most");
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -240,8 +249,7 @@ __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) m.sbuf[i * T + t] = v[i];
     __syncthreads();
-    int failed = 0;
-    if constexpr (CHECK) failed = *m.fail;  // behind the barrier: the same in every thread
+    bool met = true;
     if (wid < NV) {
         ff y[8];
 #pragma unroll
@@ -267,21 +275,24 @@ __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
     if (alone) __syncthreads();
     if constexpr (ALL && T == 512) {
         if (wid < NV) {
-            if (!alone && !mbarrier_wait(m.bar + bar, phase)) *m.fail = 1;
-            ff y = q < m.cs ? m.slots[base + wid * 16 + q] : ff_zero();
+            ff y = ff_zero();
+            if (alone || mbarrier_wait(m.bar + bar, phase, m.limit)) {
+                if (q < m.cs) y = m.slots[base + wid * 16 + q];
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1)
-                if ((unsigned)o < m.width) ff_shfl_merge(y, o);
+                for (int o = 8; o > 0; o >>= 1)
+                    if ((unsigned)o < m.width) ff_shfl_merge(y, o);
+            } else {
+                *m.fail = 1;
+                y = ff{__uint_as_float(0x7fffffffu), 0.0f};  // NaN: look at fail
+            }
             if (lane == 0) m.res[wid] = y;
         }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = m.res[i];
+        if (v[0].hi != v[0].hi) met = *m.fail == 0;
     } else if (ALL || wid == 0) {
-        if (!alone && !mbarrier_wait(m.bar + bar, phase)) {
-            if constexpr (ALL) *m.fail = 1;
-            else failed = 1;
-        }
+        if (!alone) met = mbarrier_wait(m.bar + bar, phase, m.limit);
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = q < m.cs ? m.slots[base + i * 16 + q] : ff_zero();
 #pragma unroll
@@ -292,7 +303,7 @@ __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = ff_norm(v[i]);
-    return failed == 0;
+    return met;
 }
 
 __device__ __forceinline__ float ld_shared_f32(uint32_t addr) {

@@ -131,16 +131,16 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
     }
     ff acc[3] = {cluster_merge<T>(arr), cluster_merge<T>(arz), cluster_merge<T>(abb)};
     cluster_begin(meet);
-    cluster_reduce<3, T, true, false>(acc, meet);
+    bool met = cluster_reduce<3, T, true, false>(acc, meet);
     ff rr = acc[0], rz = acc[1];
     const ff thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * ff_to_double(rr))));
-    if (me == 0 && t == 0) {
+    if (me == 0 && t == 0 && met) {
         a.stats->initial_residual = sqrt(ff_to_double(rr));
         a.stats->rhs_norm = sqrt(ff_to_double(acc[2]));
     }
     float bf = 0.0f;
     int k = 0, status = WCFD_OK;
-    while (k < a.maxiter && ff_gt(rr, thr2)) {
+    while (met && k < a.maxiter && ff_gt(rr, thr2)) {
         // p = z + beta p_old (own row and each neighbour) ; q = A p ; p.q.  The gathers of GR rows
         // are issued before the first is used.
         ff apq[NA];
@@ -192,10 +192,8 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
         }
         ff accq[1] = {cluster_merge<T>(apq)};
-        if (!cluster_reduce<1, T, true, false, true>(accq, meet)) {
-            status = WCFD_BARRIER_TIMEOUT;
-            break;
-        }
+        met = cluster_reduce<1, T, true, false>(accq, meet);
+        if (!met) break;
         if (accq[0].hi == 0.0f) {
             status = WCFD_KRYLOV_BREAKDOWN;
             break;
@@ -222,7 +220,8 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
         }
         ff acc2[2] = {cluster_merge<T>(arr), cluster_merge<T>(arz)};
-        cluster_reduce<2, T, true, false>(acc2, meet);
+        met = cluster_reduce<2, T, true, false>(acc2, meet);
+        if (!met) break;
         rr = acc2[0];
         bf = rz.hi != 0.0f ? ff_div_to_float(acc2[1], rz) : 0.0f;
         rz = acc2[1];
@@ -231,15 +230,15 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
         const int l = cluster_row<T>(t, u);
-        if (l < nloc) a.x[row0 + l] = xr[u];
+        if (met && l < nloc) a.x[row0 + l] = xr[u];
     }
     cluster_end(meet);
     if (me == 0 && t == 0) {
-        if (*meet.fail) status = WCFD_BARRIER_TIMEOUT;
+        if (!met) status = WCFD_BARRIER_TIMEOUT;
         if (status == WCFD_OK && !ff_le(rr, thr2)) status = WCFD_NOT_CONVERGED;
         a.stats->iterations = k;
         a.stats->status = status;
-        a.stats->residual = sqrt(ff_to_double(rr));
+        a.stats->residual = met ? sqrt(ff_to_double(rr)) : -1.0;
     }
 }
 
@@ -312,6 +311,48 @@ __global__ void __launch_bounds__(kBiClusterBlock, 1) bicgstab_cluster_batched(c
     const BiSystem sys{c.mom.diag, c.mom.off, c.mom.rhs, c.mesh.ell_col, c.mesh.ell_dcol, c.hbya, c.mesh.n_cells, c.prm.maxiter, false,
                        c.prm.atol_u * c.prm.atol_u, c.prm.rtol_u * c.prm.rtol_u, c.stats + 0};
     bicgstab_cluster_body<W, SMEM>(sys, c.ws_u.vec, (c.mesh.n_cells + cs_req - 1) / cs_req, cap);
+}
+
+// Self-check of the cluster's meetings: `reductions` sums of two values against their closed form
+// in every thread that gets them.  Before reduction `at` CTA `who` sleeps delay_ns (0: nobody is
+// late) or, with delay_ns < 0, leaves, so that the others' waits run out: a failure made without a
+// fault.  status[CTA]: 0, WCFD_BARRIER_TIMEOUT when the CTA gave up, -1 for wrong sums, -2 when its
+// threads disagree about having given up.  Waits give up after limit_ns.
+template <int T, bool ALL>
+__global__ void __launch_bounds__(T, 1) cluster_check_kernel(int reductions, int who, int at, long long delay_ns, long long limit_ns,
+                                                            int* __restrict__ status) {
+    __shared__ __align__(16) ClusterShared<T, 3> meeting;
+    __shared__ int s_met;
+    const int t = threadIdx.x;
+    ClusterMeet meet = cluster_meet(meeting, (uint64_t)limit_ns);
+    const bool odd = (int)meet.me == who;
+    const double n = (double)(T * meet.cs);
+    bool met = true, right = true;
+    cluster_begin(meet);
+    for (int i = 0; i < reductions && met; ++i) {
+        if (odd && i == at) {
+            if (delay_ns < 0) break;
+            const uint64_t t0 = global_ns();
+            for (int s = 0; s < 10000000 && global_ns() - t0 < (uint64_t)delay_ns; ++s) __nanosleep(100);
+            __syncthreads();
+        }
+        ff v[2] = {ff{(float)(meet.me * T + t + 1), 0.0f}, ff{(float)i, 0.0f}};
+        met = cluster_reduce<2, T, ALL, false>(v, meet);
+        if ((ALL || t == 0) && met) right = right && ff_to_double(v[0]) == 0.5 * n * (n + 1.0) && ff_to_double(v[1]) == n * i;
+        if constexpr (!ALL) {
+            if (t == 0) s_met = met;
+            __syncthreads();
+            met = s_met != 0;
+            __syncthreads();
+        }
+    }
+    const int went_on = __syncthreads_count(met), all_right = __syncthreads_and(right);
+    cluster_end(meet);
+    if (t == 0) status[meet.me] = went_on != 0 && went_on != T ? -2 : !all_right ? -1 : went_on ? WCFD_OK : WCFD_BARRIER_TIMEOUT;
+}
+const void* cluster_check_kernel_for(int T, bool all) {
+    if (T == 256) return all ? (const void*)cluster_check_kernel<256, true> : (const void*)cluster_check_kernel<256, false>;
+    return all ? (const void*)cluster_check_kernel<512, true> : (const void*)cluster_check_kernel<512, false>;
 }
 
 // dynamic shared memory of a CTA of R rows with everything in it, and the most rows that fit

@@ -366,7 +366,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         sc.k = -1;
         sc.status = met0 ? WCFD_OK : WCFD_BARRIER_TIMEOUT;
         sc.go = met0;
-        if (me == 0) {
+        if (me == 0 && met0) {
             a.stats->initial_residual = sqrt(rr0);
             a.stats->rhs_norm = sqrt(ff_to_double(red[2]));
         }
@@ -486,7 +486,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         if (st == WCFD_OK && !ff_le(sc.rr, sc.thr2)) st = WCFD_NOT_CONVERGED;
         a.stats->iterations = sc.k < 0 ? 0 : sc.k;
         a.stats->status = st;
-        a.stats->residual = sqrt(ff_to_double(sc.rr));
+        a.stats->residual = st == WCFD_BARRIER_TIMEOUT ? -1.0 : sqrt(ff_to_double(sc.rr));
     }
 }
 
