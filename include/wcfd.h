@@ -201,12 +201,12 @@ const char* wcfd_last_error(void);
  * WCFD_BARRIER_TIMEOUT), [1] 1 if a block received wrong sums, [2] blocks in the grid. */
 int wcfd_grid_barrier_check(int32_t skip_block, int32_t phases, int32_t* result, void* stream);
 /* Self-check of the meetings of the cluster-resident solvers: `reductions` sums over a cluster of
- * `ctas` CTAs (a power of two, 2..16) of 256 or 512 threads, in every thread (every_warp) or in
- * thread 0, against their closed form.  CTA `who` (-1: none) sleeps delay_ns before reduction `at` or, with
- * delay_ns < 0, leaves there; waits give up after limit_ns.  Synchronizes the stream.  result (host, one
- * per CTA): WCFD_OK, WCFD_BARRIER_TIMEOUT when its waits gave up, -1 wrong sums, -2 threads of one CTA
- * that disagree about having given up. */
-int wcfd_cluster_meeting_check(int32_t ctas, int32_t threads, int32_t every_warp, int32_t reductions, int32_t who,
+ * `ctas` CTAs (a power of two, 2..16) of 256 or 512 threads against their closed form; form 0: for
+ * thread 0, 1: for every thread, 2: for thread 0 with a barrier and a gather between them.  CTA `who`
+ * (-1: none) sleeps delay_ns before reduction `at` or, with delay_ns < 0, leaves there; waits give up after
+ * limit_ns.  Synchronizes the stream.  result (host, one per CTA): WCFD_OK, WCFD_BARRIER_TIMEOUT when a
+ * CTA's waits gave up, -1 wrong values, -2 threads of the CTA that disagree about having given up. */
+int wcfd_cluster_meeting_check(int32_t ctas, int32_t threads, int32_t form, int32_t reductions, int32_t who,
                                int32_t at, int64_t delay_ns, int64_t limit_ns, int32_t* result, void* stream);
 /* floats of wcfd_krylov_ws.vec needed for a C-row system with ncomp components */
 int64_t     wcfd_krylov_workspace_floats(int32_t n_cells, int32_t ncomp);

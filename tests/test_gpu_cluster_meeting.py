@@ -8,7 +8,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 TIMEOUT = 5
-FORMS = [(256, 1), (512, 1), (256, 0), (512, 0)]   # the CG's two, the batched CG's, the BiCGSTAB's
+# the CG's two, the BiCGSTAB's, the batched CG's two
+FORMS = [(256, 1), (512, 1), (512, 0), (256, 2), (512, 2)]
 
 
 @pytest.fixture(scope="module", autouse=True)
@@ -37,9 +38,18 @@ def test_sums_are_exact(ctas, form):
 @pytest.mark.parametrize("ctas,who,at", [(2, 0, 0), (2, 1, 3), (8, 5, 2), (16, 15, 1)])
 def test_a_cta_that_leaves_ends_the_others_waits(ctas, who, at, form):
     got = _check(ctas, form, 6, who, at, -1, 20_000)
-    assert [s for c, s in enumerate(got) if c != who] == [TIMEOUT] * (ctas - 1)
+    assert got == [TIMEOUT] * ctas
     assert _check(ctas, form, 10) == [0] * ctas
     assert float(torch.arange(1000, device="cuda", dtype=torch.float32).sum()) == 499500.0
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("ctas,who,at", [(2, 1, 0), (4, 0, 2), (8, 3, 5), (16, 7, 3)])
+def test_a_cta_that_comes_late_learns_that_the_others_left(ctas, who, at, form):
+    """The late CTA finds every total of the reduction it missed: it must not go on past the others' end,
+    at a barrier in its loop, in its next reduction or (at = 5, the last) at its own end."""
+    assert _check(ctas, form, 6, who, at, 30_000, 5_000) == [TIMEOUT] * ctas
+    assert _check(ctas, form, 10) == [0] * ctas
 
 
 @pytest.mark.parametrize("form", FORMS)
@@ -49,6 +59,6 @@ def test_threads_of_a_cta_agree_when_the_last_total_lands_as_time_runs_out(form)
     seen = set()
     for k in range(120):
         got = _check(4, form, 6, 1, 2, 250 + k, 300)
-        assert all(s in (0, TIMEOUT) for s in got), (k, got)
-        seen.add(tuple(got))
-    assert (0, 0, 0, 0) in seen and any(TIMEOUT in s for s in seen)
+        assert got in ([0] * 4, [TIMEOUT] * 4), (k, got)
+        seen.add(got[0])
+    assert seen == {0, TIMEOUT}

@@ -416,15 +416,16 @@ int wcfd_grid_barrier_check(int32_t skip_block, int32_t phases, int32_t* result,
     return rc;
 }
 
-int wcfd_cluster_meeting_check(int32_t ctas, int32_t threads, int32_t every_warp, int32_t reductions, int32_t who, int32_t at,
+int wcfd_cluster_meeting_check(int32_t ctas, int32_t threads, int32_t form, int32_t reductions, int32_t who, int32_t at,
                                int64_t delay_ns, int64_t limit_ns, int32_t* result, void* stream) {
-    RET_IF(!result || ctas < 2 || ctas > 16 || (ctas & (ctas - 1)) || (threads != 256 && threads != 512), WCFD_ERR_ARGUMENT,
-           "2 to 16 CTAs (a power of two) of 256 or 512 threads, and a result array");
+    RET_IF(!result || ctas < 2 || ctas > 16 || (ctas & (ctas - 1)) || (threads != 256 && threads != 512) ||
+               form < 0 || form > 2, WCFD_ERR_ARGUMENT,
+           "2 to 16 CTAs (a power of two) of 256 or 512 threads, form 0..2 and a result array");
     RET_IF(reductions < 1 || reductions > 100000 || who < -1 || who >= ctas || at < 0, WCFD_ERR_ARGUMENT, "bad reductions, who or at");
     RET_IF(delay_ns > 1000000000 || limit_ns < 1000 || limit_ns > 1500000000, WCFD_ERR_ARGUMENT,
            "a delay of at most 1 s, a limit of 1 us to 1.5 s");
     cudaStream_t st = S(stream);
-    const void* fn = cluster_check_kernel_for(threads, every_warp != 0);
+    const void* fn = cluster_check_kernel_for(threads, form);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(threads);

@@ -125,18 +125,24 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
 // after a block barrier behind all its reads and writes of the pass, and a CTA goes on when it has
 // every CTA's.  A cluster of one CTA needs block barriers only.  Waits are bounded.
 constexpr int kClusterSums = 3;
+constexpr unsigned kNobodyGone = ~0u;
+struct ClusterFailure {
+    int own;              // a wait of this CTA gave up (reductions of 512 threads for every thread)
+    unsigned gone;        // a CTA that gave up in this reduction leaves at the next barrier of the cluster, or kNobodyGone
+    unsigned gave_up[2];  // threads of this CTA that gave up on a mbarrier
+};
 template <int T, int SUMS>
 struct ClusterShared {
     ff slots[2 * kClusterSums * 16];  // [parity][sum][CTA]
     ff sbuf[SUMS * T];
     ff res[kClusterSums];
     unsigned long long bar[2];  // by parity
-    int fail;
+    ClusterFailure failure;
 };
 struct ClusterMeet {
     ff *slots, *sbuf, *res;
     uint32_t bar, peer_slots, peer_bar;  // own mbarriers; slots and mbarriers of CTA `lane`
-    volatile int* fail;                  // a wait of this CTA gave up (ALL with 512 threads)
+    ClusterFailure* failure;
     unsigned n, me, cs, width;           // reductions so far; width: 2^k >= cs
     uint64_t limit;                      // of a wait, ns
 };
@@ -156,13 +162,16 @@ __device__ __forceinline__ bool mbarrier_try(uint32_t bar, unsigned parity) {
 // mbarrier expect kGiveUpBytes that nobody sends and looks again.  Either the phase was complete before
 // that, and then every thread sees it (and the next phase of this mbarrier is the one that cannot
 // complete), or it never completes.  So a warp that goes on and a warp that leaves cannot part.
-// The threads of a block add less than the 2^20 - 1 bytes that an mbarrier counts.
+// The threads of a block add less than the 2^20 - 1 bytes that an mbarrier counts, and are counted in
+// gave_up (null: a thread that waits alone and may just stop).
 constexpr unsigned kGiveUpBytes = 512;  // more than the totals of a reduction (16 CTAs x 3 sums x 8)
-__device__ __forceinline__ bool mbarrier_wait(uint32_t bar, unsigned parity, uint64_t limit) {
+__device__ __forceinline__ bool mbarrier_wait(uint32_t bar, unsigned parity, uint64_t limit, unsigned* gave_up) {
     if (mbarrier_try(bar, parity)) return true;
     const uint64_t t0 = global_ns();
     while (!mbarrier_try(bar, parity)) {
         if (global_ns() - t0 <= limit) continue;
+        if (!gave_up) return false;
+        atomicAdd(gave_up, 1u);
         asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(kGiveUpBytes) : "memory");
         return mbarrier_try(bar, parity);
     }
@@ -177,7 +186,7 @@ __device__ __forceinline__ ClusterMeet cluster_meet(ClusterShared<T, SUMS>& s, u
     m.slots = s.slots;
     m.sbuf = s.sbuf;
     m.res = s.res;
-    m.fail = &s.fail;
+    m.failure = &s.failure;
     m.bar = (uint32_t)__cvta_generic_to_shared(s.bar);
     m.n = 0;
     m.me = cluster_rank();
@@ -188,7 +197,7 @@ __device__ __forceinline__ ClusterMeet cluster_meet(ClusterShared<T, SUMS>& s, u
     m.peer_slots = map_rank(s.slots, peer);
     m.peer_bar = map_rank(s.bar, peer);
     if (threadIdx.x == 0) {
-        s.fail = 0;
+        s.failure = ClusterFailure{0, kNobodyGone, {0u, 0u}};
         for (int i = 0; i < 2; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(m.bar + 8 * i), "r"(1u) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -198,8 +207,29 @@ __device__ __forceinline__ ClusterMeet cluster_meet(ClusterShared<T, SUMS>& s, u
 __device__ __forceinline__ void cluster_begin(const ClusterMeet& m) {
     if (m.cs > 1) cluster_sync_all();
 }
-__device__ __forceinline__ void cluster_end(const ClusterMeet& m) {
-    if (m.cs > 1) cluster_sync_all();
+// A barrier of the cluster inside a solve's loop, behind the same reduction in every CTA.  False when a
+// CTA gave up in that reduction and stands in cluster_end: it leaves now, so this CTA leaves too, without
+// cluster_end and without touching another CTA.  The same answer in every thread: a CTA that gives up
+// later notes a later reduction.
+__device__ __forceinline__ bool cluster_sync_met(const ClusterMeet& m) {
+    cluster_sync_all();
+    return *reinterpret_cast<volatile unsigned*>(&m.failure->gone) != m.n;
+}
+// Every thread, met: no wait of this CTA gave up.  Returns whether none of the cluster's did.  A CTA that
+// gave up tells the others before it arrives, and goes when the totals still on their way to it have landed.
+__device__ __forceinline__ bool cluster_end(const ClusterMeet& m, bool met) {
+    if (m.cs == 1) return met;
+    if (!met && threadIdx.x < m.cs)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_rank(&m.failure->gone, threadIdx.x)), "r"(m.n) : "memory");
+    cluster_sync_all();
+    if (!met && threadIdx.x == 0) {
+        const unsigned p = (m.n - 1) & 1u;
+        asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(m.bar + 8u * p),
+                     "r"(m.failure->gave_up[p] * kGiveUpBytes)
+                     : "memory");
+        mbarrier_wait(m.bar + 8u * p, ((m.n - 1) >> 1) & 1u, m.limit, nullptr);
+    }
+    return *reinterpret_cast<volatile unsigned*>(&m.failure->gone) == kNobodyGone;
 }
 
 // Row of thread t's u-th in a CTA of T = 256 or 512 threads, and the number of accumulators it
@@ -276,23 +306,23 @@ __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
     if constexpr (ALL && T == 512) {
         if (wid < NV) {
             ff y = ff_zero();
-            if (alone || mbarrier_wait(m.bar + bar, phase, m.limit)) {
+            if (alone || mbarrier_wait(m.bar + bar, phase, m.limit, &m.failure->gave_up[(m.n - 1) & 1u])) {
                 if (q < m.cs) y = m.slots[base + wid * 16 + q];
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1)
                     if ((unsigned)o < m.width) ff_shfl_merge(y, o);
             } else {
-                *m.fail = 1;
-                y = ff{__uint_as_float(0x7fffffffu), 0.0f};  // NaN: look at fail
+                *reinterpret_cast<volatile int*>(&m.failure->own) = 1;
+                y = ff{__uint_as_float(0x7fffffffu), 0.0f};  // NaN: look at failure
             }
             if (lane == 0) m.res[wid] = y;
         }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = m.res[i];
-        if (v[0].hi != v[0].hi) met = *m.fail == 0;
+        if (v[0].hi != v[0].hi) met = *reinterpret_cast<volatile int*>(&m.failure->own) == 0;
     } else if (ALL || wid == 0) {
-        if (!alone) met = mbarrier_wait(m.bar + bar, phase, m.limit);
+        if (!alone) met = mbarrier_wait(m.bar + bar, phase, m.limit, &m.failure->gave_up[(m.n - 1) & 1u]);
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = q < m.cs ? m.slots[base + i * 16 + q] : ff_zero();
 #pragma unroll

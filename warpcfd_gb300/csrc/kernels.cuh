@@ -85,7 +85,7 @@ struct CgKernel {
 CgKernel cg_kernel_for(int W, int rows);
 size_t cg_chunk_bytes(int W);  // shared memory of a chunk's column offsets
 const void* barrier_check_kernel_ptr();
-const void* cluster_check_kernel_for(int T, bool all);
+const void* cluster_check_kernel_for(int T, int form);
 const void* bicgstab_kernel_for(int W, bool resident);
 size_t bicgstab_row_bytes(int W);  // shared memory of a row of the resident form
 const void* cg_cluster_kernel_for(int W, int R);

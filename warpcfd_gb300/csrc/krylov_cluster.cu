@@ -232,7 +232,7 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
         const int l = cluster_row<T>(t, u);
         if (met && l < nloc) a.x[row0 + l] = xr[u];
     }
-    cluster_end(meet);
+    met = cluster_end(meet, met);
     if (me == 0 && t == 0) {
         if (!met) status = WCFD_BARRIER_TIMEOUT;
         if (status == WCFD_OK && !ff_le(rr, thr2)) status = WCFD_NOT_CONVERGED;
@@ -285,7 +285,10 @@ __device__ __forceinline__ void bicgstab_cluster_body(const BiSystem& sys, float
     auto run = [&](auto& net, float* own) {
         net.meet = cluster_meet(meeting);
         bicgstab_body<W, T, SMEM>(sys, net, sc, own, cap, row0, nloc, me == 0);
-        cluster_end(net.meet);
+        if (!cluster_end(net.meet, sc.status != WCFD_BARRIER_TIMEOUT) && me == 0 && threadIdx.x == 0) {
+            sys.stats->status = WCFD_BARRIER_TIMEOUT;
+            sys.stats->residual = -1.0;
+        }
     };
     if constexpr (SMEM) {
         BiShared<T> net(records, cap, R);
@@ -314,22 +317,31 @@ __global__ void __launch_bounds__(kBiClusterBlock, 1) bicgstab_cluster_batched(c
 }
 
 // Self-check of the cluster's meetings: `reductions` sums of two values against their closed form
-// in every thread that gets them.  Before reduction `at` CTA `who` sleeps delay_ns (0: nobody is
-// late) or, with delay_ns < 0, leaves, so that the others' waits run out: a failure made without a
-// fault.  status[CTA]: 0, WCFD_BARRIER_TIMEOUT when the CTA gave up, -1 for wrong sums, -2 when its
-// threads disagree about having given up.  Waits give up after limit_ns.
-template <int T, bool ALL>
+// in every thread that gets them: in every thread (FORM 1, as the CG), in thread 0 (0, the BiCGSTAB; 2,
+// the batched CG, which also meets at a barrier and gathers a word of another CTA before each reduction).
+// Before reduction `at` CTA `who` sleeps delay_ns (0: nobody is late) or, with delay_ns < 0, leaves, so that
+// the others' waits run out: a failure made without a fault.  status[CTA]: 0, WCFD_BARRIER_TIMEOUT when a
+// CTA gave up, -1 for wrong values, -2 when this CTA's threads disagree.  Waits give up after limit_ns.
+template <int T, int FORM>
 __global__ void __launch_bounds__(T, 1) cluster_check_kernel(int reductions, int who, int at, long long delay_ns, long long limit_ns,
                                                             int* __restrict__ status) {
+    constexpr bool ALL = FORM == 1;
     __shared__ __align__(16) ClusterShared<T, 3> meeting;
     __shared__ int s_met;
+    __shared__ float s_word;
     const int t = threadIdx.x;
     ClusterMeet meet = cluster_meet(meeting, (uint64_t)limit_ns);
     const bool odd = (int)meet.me == who;
     const double n = (double)(T * meet.cs);
-    bool met = true, right = true;
+    bool met = true, right = true, stay = true;
     cluster_begin(meet);
     for (int i = 0; i < reductions && met; ++i) {
+        if constexpr (FORM == 2) {
+            if (t == 0) s_word = (float)i;
+            stay = cluster_sync_met(meet);
+            if (!stay) break;
+            right = right && ld_cluster_f32(map_rank(&s_word, (meet.me + 1) % meet.cs)) == (float)i;
+        }
         if (odd && i == at) {
             if (delay_ns < 0) break;
             const uint64_t t0 = global_ns();
@@ -346,13 +358,20 @@ __global__ void __launch_bounds__(T, 1) cluster_check_kernel(int reductions, int
             __syncthreads();
         }
     }
-    const int went_on = __syncthreads_count(met), all_right = __syncthreads_and(right);
-    cluster_end(meet);
-    if (t == 0) status[meet.me] = went_on != 0 && went_on != T ? -2 : !all_right ? -1 : went_on ? WCFD_OK : WCFD_BARRIER_TIMEOUT;
+    const int went_on = __syncthreads_count(met && stay), all_right = __syncthreads_and(right);
+    const bool all_met = stay && cluster_end(meet, met);
+    if (t == 0)
+        status[meet.me] = went_on != 0 && went_on != T ? -2 : !all_right ? -1 : all_met ? WCFD_OK : WCFD_BARRIER_TIMEOUT;
 }
-const void* cluster_check_kernel_for(int T, bool all) {
-    if (T == 256) return all ? (const void*)cluster_check_kernel<256, true> : (const void*)cluster_check_kernel<256, false>;
-    return all ? (const void*)cluster_check_kernel<512, true> : (const void*)cluster_check_kernel<512, false>;
+const void* cluster_check_kernel_for(int T, int form) {
+    switch (form + (T == 512 ? 3 : 0)) {
+        case 0: return (const void*)cluster_check_kernel<256, 0>;
+        case 1: return (const void*)cluster_check_kernel<256, 1>;
+        case 2: return (const void*)cluster_check_kernel<256, 2>;
+        case 3: return (const void*)cluster_check_kernel<512, 0>;
+        case 4: return (const void*)cluster_check_kernel<512, 1>;
+        default: return (const void*)cluster_check_kernel<512, 2>;
+    }
 }
 
 // dynamic shared memory of a CTA of R rows with everything in it, and the most rows that fit

@@ -372,6 +372,7 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         }
     }
     __syncthreads();  // the reduction also published u0 to every CTA
+    bool stay = true;
     while (sc.go) {
         const float af = sc.af, bf = sc.bf;
         // (1) s = w + beta s ; p = u + beta p ; x += alpha p ; r -= alpha s ; u = M r
@@ -392,8 +393,10 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
                     ub[cluster_row<T>(t0, u)] = ur[u];
                 }
             }
-            if (meet.cs > 1) cluster_sync_all();  // every CTA's new u, visible to the cluster
+            // every CTA's new u, visible to the cluster
+            if (meet.cs > 1) stay = cluster_sync_met(meet);
             else __syncthreads();
+            if (!stay) break;
         }
         // (2) w = A u ; r.r ; r.u ; w.u.  The gathers of GR rows are issued before the first is used.
 #pragma unroll
@@ -475,18 +478,19 @@ __device__ __forceinline__ void cg1m_cluster_body(const KrylovArgs& a, int R) {
         }
         __syncthreads();
     }
+    bool met = stay && sc.status != WCFD_BARRIER_TIMEOUT;
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
         const int l = cluster_row<T>(t0, u);
-        if (l < nloc) a.x[row0 + l] = xr[u];
+        if (met && l < nloc) a.x[row0 + l] = xr[u];
     }
-    cluster_end(meet);
+    if (stay) met = cluster_end(meet, met);
     if (me == 0 && t0 == 0) {
-        int st = sc.status;
+        int st = met ? sc.status : WCFD_BARRIER_TIMEOUT;
         if (st == WCFD_OK && !ff_le(sc.rr, sc.thr2)) st = WCFD_NOT_CONVERGED;
         a.stats->iterations = sc.k < 0 ? 0 : sc.k;
         a.stats->status = st;
-        a.stats->residual = st == WCFD_BARRIER_TIMEOUT ? -1.0 : sqrt(ff_to_double(sc.rr));
+        a.stats->residual = met ? sqrt(ff_to_double(sc.rr)) : -1.0;
     }
 }
 
