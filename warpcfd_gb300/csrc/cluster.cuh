@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "wait_clock.cuh"
 
 namespace wcfd {
 
@@ -157,7 +158,7 @@ __device__ __forceinline__ bool mbarrier_try(uint32_t bar, unsigned parity) {
         : "memory");
     return done != 0;
 }
-// Wait for the phase of one of this CTA's mbarriers, `limit` ns at most.  Every thread of the CTA that
+// Wait for the phase of one of this CTA's mbarriers, `limit` ns of polling at most.  Every thread of the CTA that
 // waits for a phase gets the same answer, whichever gives up first: a thread whose time is up makes the
 // mbarrier expect kGiveUpBytes that nobody sends and looks again.  Either the phase was complete before
 // that, and then every thread sees it (and the next phase of this mbarrier is the one that cannot
@@ -167,9 +168,9 @@ __device__ __forceinline__ bool mbarrier_try(uint32_t bar, unsigned parity) {
 constexpr unsigned kGiveUpBytes = 512;  // more than the totals of a reduction (16 CTAs x 3 sums x 8)
 __device__ __forceinline__ bool mbarrier_wait(uint32_t bar, unsigned parity, uint64_t limit, unsigned* gave_up) {
     if (mbarrier_try(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
+    WaitClock clock(global_ns());
     while (!mbarrier_try(bar, parity)) {
-        if (global_ns() - t0 <= limit) continue;
+        if (!clock.over(global_ns(), limit)) continue;
         if (!gave_up) return false;
         atomicAdd(gave_up, 1u);
         asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(kGiveUpBytes) : "memory");
