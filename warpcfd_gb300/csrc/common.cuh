@@ -325,7 +325,8 @@ __device__ __forceinline__ bool grid_reduce(const GridCtl& g, ff (&acc)[NV], ff*
             unsigned spins = 0;
             uint64_t t0 = 0;
             for (;;) {
-                if ((int)(ld_acquire(g.ctr) - target) >= 0) {  // one address: the same answer in every lane
+                // the warp decides as one: its lanes' loads may be served at different times
+                if (__all_sync(0xffffffffu, (int)(ld_acquire(g.ctr) - target) >= 0)) {
                     unsigned long long tag[NV][POLL];
                     bool all = true;
 #pragma unroll
