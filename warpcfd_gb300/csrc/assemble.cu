@@ -71,6 +71,16 @@ __device__ __forceinline__ void explicit_internal_terms(const wcfd_mesh& m, cons
     }
 }
 
+// Where the j-th off-diagonal of row c goes.  An internal face that a mesh has no place for (a slot that its
+// slot_mask does not name, or more of them than ell_width: wcfd_check_mesh refuses such a mesh) goes to
+// the row's right-hand side, which the same thread writes last: a selected address, not a branch around
+// the store, which moved the coefficient's rounding in the batched kernels.
+__device__ __forceinline__ float* coefficient_place(const wcfd_mesh& m, const wcfd_system& sys, unsigned bits, int f, int j, int c,
+                                                    int ncomp) {
+    const bool has = j < m.ell_width && (bits == 0u || ((bits >> f) & 1u));
+    return has ? sys.off + (size_t)j * m.n_cells + c : sys.rhs + (size_t)ncomp * c;
+}
+
 // XT: the opt-in explicit internal terms are compiled in (their code raises the kernel from
 // 32 to 48 registers, so the default instantiation leaves it out)
 template <bool XT>
@@ -132,7 +142,7 @@ __device__ __forceinline__ void momentum_assemble_body(const wcfd_mesh& m, const
                 w1 = md > 0.0f ? mn : 0.0f;
             }
             dsum += w0 + dcoef;
-            sys.off[(size_t)j * C + c] = w1 - dcoef;
+            *coefficient_place(m, sys, bits, f, j, c, 3) = w1 - dcoef;
             ++j;
             if (XT && prm.explicit_terms)
                 explicit_internal_terms(m, s, k, owner_side, md, nu, prm.explicit_terms, 0, 3, b, 1.0f, -1.0f);
@@ -268,7 +278,7 @@ __device__ __forceinline__ void pressure_assemble_body(const wcfd_mesh& m, const
         const float coef = cfs[f];
         if (N >= 0) {
             d -= coef;
-            sys.off[(size_t)j * C + c] = ref ? 0.0f : coef;
+            *coefficient_place(m, sys, bits, f, j, c, 1) = ref ? 0.0f : coef;
             ++j;
             if (XT && (prm.explicit_terms & 4))  // opt-in non-orthogonal explicit part (see momentum)
                 explicit_internal_terms(m, s, k, sk >= 0, 0.0f, rua_faces[k], 4, 3, 1, &b, 0.0f, 1.0f);

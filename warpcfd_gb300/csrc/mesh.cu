@@ -476,7 +476,8 @@ int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 //   [2] a cell slot that is not null and names a face outside [0, K)
 //   [3] a cell slot whose face does not have this cell on the side the slot says
 //   [4] an off-diagonal column outside [0, C), or (with ell_dcol) an offset that does not
-//       give the column
+//       give the column; with slot_mask in use, an internal face in a slot that it does not name,
+//       or a named slot whose column is not the neighbour (the own row: no neighbour)
 constexpr int kChecks = 5;
 
 __global__ void check_faces_kernel(wcfd_mesh m, int* __restrict__ bad) {
@@ -494,15 +495,25 @@ __global__ void check_cells_kernel(wcfd_mesh m, int* __restrict__ bad) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n_cells) return;
     const float4* slots = reinterpret_cast<const float4*>(m.cell_slot);
+    const unsigned bits = wcfd::slot_bits(m);
     for (int f = 0; f < m.faces_per_cell; ++f) {
         const int sk = __float_as_int(slots[(size_t)f * m.n_cells + c].w);
-        if (sk == wcfd::kNullSlot) continue;
         const int k = sk >= 0 ? sk : ~sk;
-        if (k < 0 || k >= m.n_faces) {
-            atomicAdd(bad + 2, 1);
-            continue;
+        int nbr = -1;  // the cell across the face
+        if (sk != wcfd::kNullSlot) {
+            if (k < 0 || k >= m.n_faces) {
+                atomicAdd(bad + 2, 1);
+                continue;
+            }
+            if ((sk >= 0 ? m.face_owner[k] : m.face_nbr[k]) != c) atomicAdd(bad + 3, 1);
+            if (m.face_nbr[k] >= 0) nbr = sk >= 0 ? m.face_nbr[k] : m.face_owner[k];
         }
-        if ((sk >= 0 ? m.face_owner[k] : m.face_nbr[k]) != c) atomicAdd(bad + 3, 1);
+        if ((bits >> f) & 1u) {
+            const int j = __popc(bits & ((1u << f) - 1u));
+            if (m.ell_col[(size_t)j * m.n_cells + c] != (nbr >= 0 ? nbr : c)) atomicAdd(bad + 4, 1);
+        } else if (bits && nbr >= 0) {
+            atomicAdd(bad + 4, 1);
+        }
     }
     for (int j = 0; j < m.ell_width; ++j) {
         const int col = m.ell_col[(size_t)j * m.n_cells + c];
@@ -524,6 +535,9 @@ int wcfd_check_mesh(const wcfd_mesh* m, int32_t* counts, void* stream) {
         return mesh_error(WCFD_ERR_ARGUMENT, "bad mesh sizes");
     if (!m->face_owner || !m->face_nbr || !m->face_brow || !m->cell_slot || !m->ell_col)
         return mesh_error(WCFD_ERR_ARGUMENT, "mesh has a null index array");
+    if (const unsigned bits = wcfd::slot_bits(*m);
+        bits >> m->faces_per_cell || (bits && __builtin_popcount(bits) != m->ell_width))
+        return mesh_error(WCFD_ERR_ARGUMENT, "slot_mask must name ell_width of the cells' slots");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int* bad = nullptr;
     if (cudaMalloc(&bad, kChecks * sizeof(int)) != cudaSuccess) MESH_CHECK("allocation");
