@@ -77,7 +77,7 @@ typedef struct wcfd_mesh {
                                      with fewer faces than F in a mixed mesh) */
     const float*   cell_volume;   /* [C]                                               */
     const int32_t* ell_col;       /* [W*C] slot-major neighbour column; padding = own row */
-    const int32_t* boundary_face; /* [B]   face id of each boundary row               */
+    const int32_t* boundary_face; /* [B]   face id of each boundary row; NULL: set_boundary_conditions walks all faces */
     const float*   face_dvec;     /* [K*4] owner->neighbour centroid vector d (internal faces)
                                      and 0; read only by the opt-in explicit internal terms
                                      (wcfd_params.explicit_terms), may be NULL otherwise */
@@ -490,7 +490,7 @@ const char* wcfd_mesh_last_error(void);
 
 /* Bounds and consistency check of a device geometry's index arrays (no reference
  * counterpart; the stand-in for a sanitizer on the gathers): face owner / neighbour in
- * range, boundary rows in range, every non-null cell slot naming a face that has the cell
+ * range, boundary rows in range and listed with their faces, every non-null cell slot naming a face that has the cell
  * on that side, every off-diagonal column in range and, with slot_mask in use, the one that its
  * slot's face says (no internal face in a slot without a place).  Each index is read only after the
  * bounds it is used under were checked.  Synchronizes the stream; counts (host, 5 ints)

@@ -75,3 +75,36 @@ def test_assembly_with_a_wrong_slot_mask_stays_in_its_array(monkeypatch, what):
     torch.cuda.synchronize()
     assert bool((off[W * C:] == 7.0).all())
     assert np.isfinite(off.cpu().numpy()).all()
+
+
+def test_boundary_list_is_checked_and_its_order_does_not_matter():
+    """set_boundary_conditions goes by the list of boundary faces: entries that are no boundary face are
+    counted and skipped, and every face gets its own row's values in whatever order the list has them."""
+    from tests.cases import cavity_bc, cavity_mesh
+    from tests.gpu_helpers import make_pair
+    from warpcfd_gb300 import _lib
+    model = make_pair(cavity_mesh(9), cavity_bc)[0]
+    faces, K = model._geo["boundary_face"], model._geo["n_faces"]
+    start = [torch.randn_like(a) for a in (model.face_values, model.face_gradients)]
+
+    def apply(lst):
+        ms = model.mesh_struct()
+        ms.boundary_face = lst.data_ptr()
+        for a, b in zip((model.face_values, model.face_gradients), start):
+            a.copy_(b)
+        _lib.call("wcfd_set_boundary_conditions", ct.byref(ms), model.bc_struct(), model.state_struct(), None)
+        torch.cuda.synchronize()
+        return _check(ms), model.face_values.clone(), model.face_gradients.clone()
+
+    (rc, c), fv, fg = apply(faces)
+    assert rc == 0 and c == [0] * 5 and not torch.equal(fv, start[0])
+    (rc, c), fv2, fg2 = apply(faces.flip(0).contiguous())
+    assert rc == _lib.WCFD_ERR_ARGUMENT and c[1] >= len(faces) - 1 and c[0] + c[2] + c[3] + c[4] == 0
+    assert torch.equal(fv, fv2) and torch.equal(fg, fg2)
+    bad = faces.clone()
+    gone = bad[[0, 3, 5]].long()
+    bad[0], bad[3], bad[5] = -1, K, int((model._geo["face_nbr"] >= 0).nonzero()[0])   # the last an internal face
+    (rc, c), fv3, fg3 = apply(bad)
+    assert rc == _lib.WCFD_ERR_ARGUMENT and c[1] == 3
+    fv[gone], fg[gone] = start[0][gone], start[1][gone]
+    assert torch.equal(fv, fv3) and torch.equal(fg, fg3)

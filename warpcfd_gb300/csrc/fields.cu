@@ -183,13 +183,17 @@ __global__ void __launch_bounds__(kBlock, WCFD_FACE_PARTIAL_MINB) face_pass_part
 // The boundary tables alone (set_boundary_conditions), a thread per boundary face: what the face
 // pass does for mask 0 and flag bit0, without walking the internal faces, which it would read
 // and write back as they are.  A few microseconds of launch against 59 us for the 4.3 M faces
-// of a 112 x 121 x 104 box.
+// of a 112 x 121 x 104 box.  The list says which faces; a face's row is face_brow's, as in the face pass,
+// whatever the list's order.
 __global__ void __launch_bounds__(kBlock) boundary_values_kernel(wcfd_mesh m, wcfd_bc bc, wcfd_state s) {
     const int b = blockIdx.x * kBlock + threadIdx.x;
     if (b >= m.n_bfaces) return;
     const int k = __ldg(m.boundary_face + b);
-    const uchar4 t = __ldg(reinterpret_cast<const uchar4*>(bc.type) + b);
-    const float4 bv = __ldg(reinterpret_cast<const float4*>(bc.value) + b);
+    if (k < 0 || k >= m.n_faces) return;
+    const int r = __ldg(m.face_brow + k);
+    if (r < 0 || r >= m.n_bfaces) return;
+    const uchar4 t = __ldg(reinterpret_cast<const uchar4*>(bc.type) + r);
+    const float4 bv = __ldg(reinterpret_cast<const float4*>(bc.value) + r);
     float4 fv = ld4(s.face_values + 4 * (size_t)k), fg = ld4(s.face_gradients + 4 * (size_t)k);
     const uint8_t tt[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll

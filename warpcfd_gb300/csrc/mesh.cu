@@ -472,7 +472,8 @@ int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 // check reads an index only after the bounds it is used under have been checked, and each
 // violation adds one to a counter per kind.
 //   [0] face owner outside [0, C) or neighbour outside [-1, C) or equal to the owner
-//   [1] boundary row of a boundary face outside [0, B)
+//   [1] boundary row of a boundary face outside [0, B); an entry of boundary_face (when given) that is
+//       no face or not the face of its row
 //   [2] a cell slot that is not null and names a face outside [0, K)
 //   [3] a cell slot whose face does not have this cell on the side the slot says
 //   [4] an off-diagonal column outside [0, C), or (with ell_dcol) an offset that does not
@@ -488,6 +489,11 @@ __global__ void check_faces_kernel(wcfd_mesh m, int* __restrict__ bad) {
     if (N < 0) {
         const int b = m.face_brow[k];
         if (b < 0 || b >= m.n_bfaces) atomicAdd(bad + 1, 1);
+    }
+    if (!m.boundary_face) return;
+    for (long long b = k; b < m.n_bfaces; b += m.n_faces) {
+        const int f = m.boundary_face[b];
+        if (f < 0 || f >= m.n_faces || m.face_brow[f] != b) atomicAdd(bad + 1, 1);
     }
 }
 
