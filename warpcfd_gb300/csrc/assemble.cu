@@ -71,16 +71,6 @@ __device__ __forceinline__ void explicit_internal_terms(const wcfd_mesh& m, cons
     }
 }
 
-// Where the j-th off-diagonal of row c goes.  An internal face that a mesh has no place for (a slot that its
-// slot_mask does not name, or more of them than ell_width: wcfd_check_mesh refuses such a mesh) goes to
-// the row's right-hand side, which the same thread writes last: a selected address, not a branch around
-// the store, which moved the coefficient's rounding in the batched kernels.
-__device__ __forceinline__ float* coefficient_place(const wcfd_mesh& m, const wcfd_system& sys, unsigned bits, int f, int j, int c,
-                                                    int ncomp) {
-    const bool has = j < m.ell_width && (bits == 0u || ((bits >> f) & 1u));
-    return has ? sys.off + (size_t)j * m.n_cells + c : sys.rhs + (size_t)ncomp * c;
-}
-
 // XT: the opt-in explicit internal terms are compiled in (their code raises the kernel from
 // 32 to 48 registers, so the default instantiation leaves it out)
 template <bool XT>
@@ -92,6 +82,11 @@ __device__ __forceinline__ void momentum_assemble_body(const wcfd_mesh& m, const
     float b[3] = {0.0f, 0.0f, 0.0f};
     int j = 0;
     const unsigned bits = slot_bits(m);
+    // The last off-diagonal slot: an internal face that a mesh has no place for (a slot that its slot_mask does
+    // not name; wcfd_check_mesh refuses such a mesh) keeps the j of the slot before, which may be one past
+    // it.  A minimum in the address: a branch around the store moved the coefficient's rounding in the batched
+    // kernels, and a selected address took 60 registers for 48 (128^3: 104 us for 96).
+    const int last = max(m.ell_width, 1) - 1;
     const float4* slots = reinterpret_cast<const float4*>(m.cell_slot);
     // Every slot's face reference first, then every face's flux, neighbour and coefficient,
     // all independent loads: a thread's chain of global-memory round trips is two deep
@@ -142,7 +137,7 @@ __device__ __forceinline__ void momentum_assemble_body(const wcfd_mesh& m, const
                 w1 = md > 0.0f ? mn : 0.0f;
             }
             dsum += w0 + dcoef;
-            *coefficient_place(m, sys, bits, f, j, c, 3) = w1 - dcoef;
+            sys.off[(size_t)min(j, last) * C + c] = w1 - dcoef;
             ++j;
             if (XT && prm.explicit_terms)
                 explicit_internal_terms(m, s, k, owner_side, md, nu, prm.explicit_terms, 0, 3, b, 1.0f, -1.0f);
@@ -249,6 +244,7 @@ __device__ __forceinline__ void pressure_assemble_body(const wcfd_mesh& m, const
     float d = 0.0f, b = 0.0f;
     int j = 0;
     const unsigned bits = slot_bits(m);
+    const int last = max(m.ell_width, 1) - 1;  // as in the momentum assembly
     const bool ref = (c == prm.ref_cell);
     const float4* slots = reinterpret_cast<const float4*>(m.cell_slot);
     // the same two-deep load structure as the momentum assembly
@@ -278,7 +274,7 @@ __device__ __forceinline__ void pressure_assemble_body(const wcfd_mesh& m, const
         const float coef = cfs[f];
         if (N >= 0) {
             d -= coef;
-            *coefficient_place(m, sys, bits, f, j, c, 1) = ref ? 0.0f : coef;
+            sys.off[(size_t)min(j, last) * C + c] = ref ? 0.0f : coef;
             ++j;
             if (XT && (prm.explicit_terms & 4))  // opt-in non-orthogonal explicit part (see momentum)
                 explicit_internal_terms(m, s, k, sk >= 0, 0.0f, rua_faces[k], 4, 3, 1, &b, 0.0f, 1.0f);
