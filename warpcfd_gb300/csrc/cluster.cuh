@@ -128,7 +128,7 @@ __device__ __forceinline__ void cluster_reduce_tree(const ff (&acc)[NV], ff (&ou
 constexpr int kClusterSums = 3;
 constexpr unsigned kNobodyGone = ~0u;
 struct ClusterFailure {
-    int own;              // a wait of this CTA gave up (reductions of 512 threads for every thread)
+    int own;              // a wait of this CTA gave up (reductions for every thread)
     unsigned gone;        // a CTA that gave up in this reduction leaves at the next barrier of the cluster, or kNobodyGone
     unsigned gave_up[2];  // threads of this CTA that gave up on a mbarrier
 };
@@ -262,8 +262,9 @@ __device__ __forceinline__ ff cluster_merge(ff (&acc)[kClusterAcc<T>]) {
 // 0 only.  Warp i merges value i over the CTA's threads (eight or sixteen per lane, pairwise,
 // then by butterfly) and sends the total to every CTA; every warp of a small CTA (ALL, T = 256),
 // warp i (ALL, T = 512) or warp 0 then merges the cs <= 16 totals.  FENCE: global memory
-// written before is visible to the cluster after.  False when the wait gave up: in every thread of
-// the CTA (ALL), else in thread 0, which owns the scalars.
+// written before is visible to the cluster after.  When the wait gave up: false in thread 0, which owns
+// the scalars (not ALL); NaN in every sum of every thread of the CTA and cluster_gave_up true (ALL), so that
+// the tests that a solver makes of its sums anyway find it.
 template <int NV, int T, bool ALL, bool FENCE>
 __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
     static_assert(NV <= kClusterSums, "three sums at most");
@@ -314,16 +315,25 @@ __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
                     if ((unsigned)o < m.width) ff_shfl_merge(y, o);
             } else {
                 *reinterpret_cast<volatile int*>(&m.failure->own) = 1;
-                y = ff{__uint_as_float(0x7fffffffu), 0.0f};  // NaN: look at failure
+                y = ff{__uint_as_float(0x7fffffffu), 0.0f};
             }
             if (lane == 0) m.res[wid] = y;
         }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = m.res[i];
-        if (v[0].hi != v[0].hi) met = *reinterpret_cast<volatile int*>(&m.failure->own) == 0;
     } else if (ALL || wid == 0) {
-        if (!alone) met = mbarrier_wait(m.bar + bar, phase, m.limit, &m.failure->gave_up[(m.n - 1) & 1u]);
+        if (!alone && !mbarrier_wait(m.bar + bar, phase, m.limit, &m.failure->gave_up[(m.n - 1) & 1u])) {
+            if constexpr (ALL) {
+                *reinterpret_cast<volatile int*>(&m.failure->own) = 1;
+                // this CTA's own total among them is long there and stays NaN
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    if (q < m.cs) m.slots[base + i * 16 + q] = ff{__uint_as_float(0x7fffffffu), 0.0f};
+            } else {
+                met = false;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = q < m.cs ? m.slots[base + i * 16 + q] : ff_zero();
 #pragma unroll
@@ -335,6 +345,11 @@ __device__ __forceinline__ bool cluster_reduce(ff (&v)[NV], ClusterMeet& m) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = ff_norm(v[i]);
     return met;
+}
+
+// after a reduction for every thread (ALL) whose sums are NaN, or after the last one
+__device__ __forceinline__ bool cluster_gave_up(const ClusterMeet& m) {
+    return *reinterpret_cast<volatile int*>(&m.failure->own) != 0;
 }
 
 __device__ __forceinline__ float ld_shared_f32(uint32_t addr) {

@@ -15,10 +15,11 @@
 //    take the same branch at every test.
 //  * The direction update p = z + beta p is evaluated inside the SpMV for the row and its
 //    neighbours, so an iteration needs two reductions.
-// Bound by the latency of its two reductions and, with many rows a CTA, by instruction issue.
+// Bound by latency: of its two reductions and, with many rows a CTA, of remote gathers and dependent
+// arithmetic with two to four warps a scheduler (16 x 2,000 rows: an instruction in 40% of the cycles).
 // Measured per iteration (1,024 threads, everything in shared memory, cluster barriers -> this
-// form): 2 CTAs x 512 rows 2.71 -> 1.40 us, 8 x 512 2.87 -> 1.49, 16 x 2,000 3.77 -> 2.35, 16 x 4,096
-// 4.69 -> 3.45 (the grid kernel: 4.59).
+// form): 2 CTAs x 512 rows 2.68 -> 1.37 us, 8 x 512 2.87 -> 1.54, 16 x 2,000 3.77 -> 2.39, 16 x 4,096
+// 4.68 -> 3.37 (the grid kernel: 4.59).
 // The arithmetic is that of cg_kernel (krylov.cu): the same Jacobi-preconditioned CG with
 // fp64-accurate dot products and the same stop test.
 #include "bicgstab.cuh"
@@ -41,7 +42,7 @@ size_t cluster_cg_smem_bytes(int R, int W) {
     return (size_t)cap * (8 + (cap > 2048 ? 4 * (size_t)W + 8 : 0));
 }
 
-// Largest R of a cluster solve: 4,096 up to width 4, 3,735 and 3,430 at 5 and 6, where the grid
+// Largest R of a cluster solve: 4,096 up to width 4, 3,811 and 3,430 at 5 and 6, where the grid
 // kernel takes over (and where the batched form's limit lies); at most what 8 x 512 threads hold.
 int cluster_cg_max_rows(int W, int optin) {
     const long long r = ((long long)optin - 26624) / (6LL * W + 24);
@@ -131,16 +132,16 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
     }
     ff acc[3] = {cluster_merge<T>(arr), cluster_merge<T>(arz), cluster_merge<T>(abb)};
     cluster_begin(meet);
-    bool met = cluster_reduce<3, T, true, false>(acc, meet);
+    cluster_reduce<3, T, true, false>(acc, meet);
     ff rr = acc[0], rz = acc[1];
     const ff thr2 = ff_norm(ff_from_double(fmax(a.atol2, a.rtol2 * ff_to_double(rr))));
-    if (me == 0 && t == 0 && met) {
+    if (me == 0 && t == 0 && !cluster_gave_up(meet)) {
         a.stats->initial_residual = sqrt(ff_to_double(rr));
         a.stats->rhs_norm = sqrt(ff_to_double(acc[2]));
     }
     float bf = 0.0f;
     int k = 0, status = WCFD_OK;
-    while (met && k < a.maxiter && ff_gt(rr, thr2)) {
+    while (k < a.maxiter && ff_gt(rr, thr2)) {  // not with a NaN
         // p = z + beta p_old (own row and each neighbour) ; q = A p ; p.q.  The gathers of GR rows
         // are issued before the first is used.
         ff apq[NA];
@@ -192,11 +193,10 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
         }
         ff accq[1] = {cluster_merge<T>(apq)};
-        met = cluster_reduce<1, T, true, false>(accq, meet);
-        if (!met) break;
-        if (accq[0].hi == 0.0f) {
-            status = WCFD_KRYLOV_BREAKDOWN;
-            break;
+        cluster_reduce<1, T, true, false>(accq, meet);
+        if (!(accq[0].hi < 0.0f || accq[0].hi > 0.0f)) {
+            if (accq[0].hi == 0.0f) status = WCFD_KRYLOV_BREAKDOWN;
+            if (accq[0].hi == 0.0f || cluster_gave_up(meet)) break;
         }
         const float af = ff_div_to_float(rz, accq[0]);
         // x += alpha p ; r -= alpha q ; z = M r ; rr ; rz
@@ -220,13 +220,13 @@ __device__ __forceinline__ void cg_cluster_body(const KrylovArgs& a, int R) {
             }
         }
         ff acc2[2] = {cluster_merge<T>(arr), cluster_merge<T>(arz)};
-        met = cluster_reduce<2, T, true, false>(acc2, meet);
-        if (!met) break;
+        cluster_reduce<2, T, true, false>(acc2, meet);
         rr = acc2[0];
         bf = rz.hi != 0.0f ? ff_div_to_float(acc2[1], rz) : 0.0f;
         rz = acc2[1];
         ++k;
     }
+    bool met = !cluster_gave_up(meet);
 #pragma unroll
     for (int u = 0; u < RPT; ++u) {
         const int l = cluster_row<T>(t, u);
@@ -350,6 +350,8 @@ __global__ void __launch_bounds__(T, 1) cluster_check_kernel(int reductions, int
         }
         ff v[2] = {ff{(float)(meet.me * T + t + 1), 0.0f}, ff{(float)i, 0.0f}};
         met = cluster_reduce<2, T, ALL, false>(v, meet);
+        if constexpr (ALL) met = v[0].hi == v[0].hi && v[1].hi == v[1].hi;
+        right = right && (!ALL || met != cluster_gave_up(meet));
         if ((ALL || t == 0) && met) right = right && ff_to_double(v[0]) == 0.5 * n * (n + 1.0) && ff_to_double(v[1]) == n * i;
         if constexpr (!ALL) {
             if (t == 0) s_met = met;
