@@ -54,11 +54,11 @@ METRIC = "cell-iterations/s"
 # (`dram__bytes_read.sum + dram__bytes_write.sum`, one capture per workload):
 #   channel   cg_cluster_kernel: 1.47 MB per launch whatever the iteration count (the
 #             system is read once into shared memory)
-#   cavity3d  cg_kernel (off-diagonals in place): 178 MB for a launch of 100 iterations (the
-#             matrix and the vectors stay in L2 and shared memory; set-up included)
+#   cavity3d  cg_kernel (off-diagonals in place): 177.6 MB for a launch of 100 iterations, 249.1 for one of
+#             174 (the set-up, and what the matrix and the vectors miss of L2 and shared memory)
 MEASURED_TRAFFIC = {
     "channel": {"per_launch": 1.473e6, "per_iteration": 0.0},
-    "cavity3d": {"per_launch": 177.6e6, "per_iteration": 0.0},
+    "cavity3d": {"per_launch": 81.0e6, "per_iteration": 0.966e6},
 }
 
 
@@ -613,8 +613,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peaks
                      else "fallback", "traffic": traffic,
-                     "traffic_note": "ncu DRAM bytes per launch of this kernel on this workload (one capture, "
-                                     "scaled by the mean iteration count)" if traffic is not None else None,
+                     "traffic_note": "ncu DRAM bytes per launch of this kernel on this workload (set-up and "
+                                     "iterations from captures, for the mean iteration count)" if traffic is not None else None,
                      "bytes_per_launch": kbytes / nl, "ms_per_launch": kms / nl,
                      "step_bytes_per_s_GBs": float(np.sum(step_bytes) / (total_ms * 1e-3) / 1e9)},
         "kernel_ms": {"bicgstab": float(bicg_ms.mean()), "cg": float(cg_ms.mean()), "step": float(step_ms.mean())},

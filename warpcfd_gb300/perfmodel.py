@@ -27,7 +27,16 @@ def cg_bytes(C: int, W: int, iters: int, col_bytes: int = 4) -> int:
     return cg_bytes_setup(C, W, col_bytes) + iters * cg_bytes_per_iteration(C, W, col_bytes)
 
 
-BICG_RESIDENT_ROWS = 152 * 227 * 1024  # over the bytes of a row: what the grid's shared memory holds
+BICG_BLOCKS, BICG_ROWS_PER_BLOCK = 152, 256  # most blocks of the grid BiCGSTAB, rows it gives a block before that
+BICG_BLOCK_BYTES = 232448 - 4176             # a block's shared memory, less what the kernel itself takes
+
+
+def bicgstab_resident(C: int, W: int) -> bool:
+    """Whether the grid BiCGSTAB keeps a block's rows in shared memory (launch_krylov, capi.cu): rows per
+    block rounded up to 32, 24 + 2 W floats a row."""
+    blocks = max(1, min(BICG_BLOCKS, -(-C // BICG_ROWS_PER_BLOCK)))
+    rows = -(-(-(-C // blocks)) // 32) * 32
+    return rows * (96 + 8 * W) <= BICG_BLOCK_BYTES
 
 
 def bicgstab_bytes_per_iteration(C: int, W: int, col_bytes: int = 4) -> int:
@@ -39,7 +48,7 @@ def bicgstab_bytes_per_iteration(C: int, W: int, col_bytes: int = 4) -> int:
     A resident system moves those; a streamed one also off/col (4 + col_bytes) W + diag 12 in
     each product, r0 12 + p 12 (w), t 12 (w), and R, V, Z 36 + r0, p, t, x 48 + x 12 (w).
     """
-    if C * (96 + 8 * W) <= BICG_RESIDENT_ROWS:
+    if bicgstab_resident(C, W):
         return C * 120
     return C * (2 * (4 + col_bytes) * W + 276)
 
