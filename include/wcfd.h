@@ -83,8 +83,9 @@ typedef struct wcfd_mesh {
                                      (wcfd_params.explicit_terms), may be NULL otherwise */
     const int16_t* ell_dcol;      /* [W*C] ell_col - row as int16, when every |ell_col - row|
                                      <= 32767 (e.g. a structured numbering), else NULL: where
-                                     the grid-cooperative CG reads columns it then streams 2
-                                     bytes per slot instead of 4 (the same columns and bits) */
+                                     the grid-cooperative CG and the streamed BiCGSTAB (grid, or
+                                     batched) read columns they then take 2 bytes per slot instead
+                                     of 4 (the same columns and bits) */
 } wcfd_mesh;
 
 /* boundary tables, one row per boundary face, columns u,v,w,p */
@@ -293,14 +294,15 @@ int wcfd_cg(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws, doub
 int wcfd_cg_refine(const wcfd_mesh* m, wcfd_system A, double* x64, float* x32, float* work, wcfd_krylov_ws ws,
                    int32_t sweeps, double inner_rtol, int32_t maxiter, wcfd_solve_stats* stats, void* stream);
 
-/* Which CG kernel wcfd_cg runs: 0 = automatic (the cluster-resident kernel when the system
+/* Which kernels wcfd_cg and wcfd_bicgstab run: 0 = automatic (the cluster-resident kernel when the system
  * fits in the shared memory of one cluster of up to 16 CTAs, else the grid-cooperative
  * kernel), 1 = always grid-cooperative, 2 = cluster-resident when it fits, 3 = as 2 with
  * the single-reduction (Chronopoulos-Gear) arrangement of CG where it fits (up to 2048
- * rows per CTA): one cluster all-reduce per iteration instead of two (its kernel takes 3.4 us
- * on a 32,000-row system, the automatic one 2.35), the same iterates as textbook CG up to rounding (which, on
- * ill-conditioned systems, moves the solution at an absolute stop by ~1e-4 relative).
- * Process-wide. */
+ * rows per CTA): one cluster all-reduce per iteration instead of two, the same iterates as
+ * textbook CG up to rounding (which, on ill-conditioned systems, moves the solution at an
+ * absolute stop by ~1e-4 relative); it was the faster one once and is not now (3.4 us an iteration
+ * on 32,000 rows, the automatic kernel 2.39).  wcfd_bicgstab follows the same switch: 1 = grid-
+ * cooperative, otherwise one cluster of up to 16 CTAs while the system fits it.  Process-wide. */
 int wcfd_set_krylov_path(int32_t path);
 int wcfd_bicgstab(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws, double atol,
                   int32_t maxiter, wcfd_solve_stats* stats, void* stream);

@@ -23,6 +23,11 @@ int batch_budget_rows(int W) {
     return cluster_cg_max_rows(W, optin);
 }
 
+// The fewest CTAs per case of at most 2,048 rows each, where the caller does not say.  Measured, us a step
+// (100 CG iterations, single-reduction form) with 1 / 2 / 4 / 8 / 16 CTAs per case:
+//   4,096 cells: one case 352 / 275 / 229 / 209 / 219, 16 cases 366 / 290 / 243 / 251 / 450, 64 cases 442 / 363 / 510 / 560 / 1,203
+//   2,048 cells: one case 234 / 224 / 207 / 208 / 220, 16 cases 240 / 229 / 212 / 238 / 439, 64 cases 268 / 256 / 273 / 498 / 1,148
+// so 2,048 rows are right where a batch fills the GPU at the largest size and cost a lone case of it a quarter.
 int pick_cluster(const wcfd_batch_dims& d) {
     const int rmax = batch_budget_rows(d.ell_width);
     for (int c = 1; c <= 16; c *= 2) {

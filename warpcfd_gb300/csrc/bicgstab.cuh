@@ -16,13 +16,13 @@
 // t are planes of the workspace.
 //
 // The operations per value are the same in every form.  Bound by the three reductions of an
-// iteration while resident (6 us of them on the grid, under 2 in a cluster), by the bytes of the
+// iteration while resident (6 us of them on the grid, about 2 in a cluster), by the bytes of the
 // matrix and about 22 floats a row beyond (128^3: 350 bytes a row and iteration, 5.0 TB/s).
 // Measured per iteration against the form with scalar vectors in the workspace and 1,024 threads
-// of one row: 1,024 rows 12.9 -> 2.2 us, 4,096 14.1 -> 2.9 (cluster); 32,000 14.5 -> 6.2, 55,000
-// tetrahedra 18.0 -> 7.9, 152,000 19.1 -> 10.6, 247,000 of width 4 25 -> 13.6 (grid, resident);
-// 864,000 76 -> 54, 128^3 172 -> 148 (streamed; without the prefetch 157, with r0, the diagonal and
-// the records prefetched too 151 to 158).
+// of one row: 1,024 rows 14.3 -> 3.7 us, 4,096 14.8 -> 4.0 (cluster); 32,000 15.4 -> 7.3, 55,000
+// tetrahedra 18.7 -> 8.3, 152,000 19.6 -> 11.8, 247,000 of width 4 25.4 -> 14.7 (grid, resident);
+// 255,000 of width 6 27.9 -> 19.8, 864,000 76 -> 54, 128^3 174 -> 148 (streamed; without the prefetch 157,
+// with r0, the diagonal and the records prefetched too 151 to 158).
 #pragma once
 #include "cluster.cuh"
 #include "common.cuh"

@@ -11,7 +11,8 @@ using namespace wcfd;
 // rows per block the grid-cooperative Krylov kernels are sized for (capped at the blocks
 // that can be co-resident)
 #ifndef WCFD_BICG_ROWS_PER_BLOCK
-#define WCFD_BICG_ROWS_PER_BLOCK 256  // 32,000 rows: 6.5 us an iteration, with 512 7.3, with 128 6.2
+#define WCFD_BICG_ROWS_PER_BLOCK 256  // us an iteration with 128 / 256 / 512 / 1,024: 32,000 rows of width 4 7.0 / 7.1 / 7.8 /
+                                      // 9.6, 32,768 of width 6 7.6 / 7.8 / 8.4 / 11.0; from 38,900 rows on 256 and 128 are the same grid
 #endif
 #ifndef WCFD_CG_ROWS_PER_BLOCK
 #define WCFD_CG_ROWS_PER_BLOCK 512
@@ -221,8 +222,11 @@ int g_krylov_path = 0;  // 0 automatic, 1 grid-cooperative only, 2 cluster-resid
 
 // the cluster CG takes the smallest cluster whose CTAs hold at most this many rows each
 // (larger systems take 16 CTAs).  Its iteration is bound by the cluster reductions, so
-// more CTAs with fewer rows per thread are faster down to ~512 rows per CTA (measured on a
-// 4,096-row system: 2,048 rows per CTA 120 us per solve, 1,024 108, 512 106, 256 113)
+// more CTAs with fewer rows per thread are faster down to 512 rows per CTA, two rows a thread.
+// Measured, us an iteration with at most 256 / 512 / 1,024 / 2,048 rows per CTA:
+//   width 4: 1,024 rows 1.46 / 1.36 / 1.44 / 1.44, 2,048 1.55 / 1.47 / 1.58 / 1.87, 4,096 1.69 / 1.54 / 1.70 / 2.01,
+//            8,192 1.70 / 1.70 / 1.78 / 2.10, 16,384 1.91 / 1.91 / 1.91 / 2.17
+//   width 6: 1,000 rows 1.67 / 1.53 / 1.72 / 1.72, 4,096 1.78 / 1.62 / 1.86 / 2.35, 8,000 1.85 / 1.85 / 1.91 / 2.49
 #ifndef WCFD_CLUSTER_ROW_CAP
 #define WCFD_CLUSTER_ROW_CAP 512
 #endif
@@ -337,12 +341,13 @@ int try_cluster_cg(const wcfd_mesh* m, wcfd_system A, float* x, double atol, int
     return launch_cluster_solve(fn, cs, threads, smem, m, A, x, nullptr, atol, rtol, maxiter, stats, st, R, "cg_cluster_kernel");
 }
 
-// rows per CTA that the cluster BiCGSTAB aims at: 4,096 rows on 16 CTAs 2.86 us an iteration, on 8 3.38
+// rows per CTA that the cluster BiCGSTAB aims at.  Measured, us an iteration with 128 / 256 / 512 / 1,024:
+//   width 4: 1,024 rows 3.53 / 3.70 / 4.38 / 5.92, 2,048 3.87 / 3.87 / 4.55 / 6.09, 4,096 4.04 / 4.04 / 4.72 / 6.26
+//   width 6: 1,000 rows 4.04 / 4.22 / 5.06 / 7.12, 4,096 4.90 / 4.90 / 5.58 / 7.63, 8,000 (16 CTAs but the last) 6.09 / 6.09 / 6.08 / 7.63
 constexpr int kBicgClusterRows = 256;
 
-// Cluster-resident BiCGSTAB under the same terms: up to 16 CTAs of about 1,000 rows.  With more rows
-// the grid kernel's 152 SMs outweigh its dearer barriers (4,096 rows: 2.9 us an iteration here, 5.8
-// there; 32,000 rows there 6.2).
+// Cluster-resident BiCGSTAB under the same terms: up to 16 CTAs of about 1,000 rows (16,384 rows of width
+// 4 6.6 us an iteration here), the most that fit; the grid kernel takes 7.1 at 32,000.
 int try_cluster_bicgstab(const wcfd_mesh* m, wcfd_system A, float* x, wcfd_krylov_ws ws, double atol, int maxiter,
                          wcfd_solve_stats* stats, cudaStream_t st, double rtol) {
     if (g_krylov_path == 1) return -1;

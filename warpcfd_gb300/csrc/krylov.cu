@@ -29,8 +29,8 @@ __device__ __forceinline__ float jacobi(float d) { return d != 0.0f ? 1.0f / d :
 
 // Krylov scalars of one block, owned by thread 0
 struct KScalars {
-    ff rr, rz, rho, alpha, omega, thr2;
-    float af, bf, of;
+    ff rr, rz, thr2;
+    float af, bf;
     int go, status, k;
 };
 

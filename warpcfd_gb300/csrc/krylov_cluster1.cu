@@ -252,9 +252,10 @@ const void* cg1_cluster_kernel_for(int W, int R) {
 // diagonals in shared memory, one 16-byte load a row at width 4).  Cycles of an iteration at
 // 4,096 rows on one CTA, 1,024 threads with everything in shared memory -> this form: update
 // 1,259 -> 788, barrier 1,116 -> 109, SpMV and products 4,082 -> 3,031, reduction 2,865 -> 1,027,
-// scalars 894 -> 940.  Bound by instruction issue (about 120 a row and iteration, half of them
-// the exact products); groups of rows that a smaller case of the batch does not have are
-// skipped whole.
+// scalars 894 -> 940.  About 120 instructions a row and iteration, half of them the exact products; one is
+// issued in 41% of the cycles, and a third of the stalls are warps at a block barrier while one of them
+// merges the sums and one thread forms the scalars.  Groups of rows that a smaller case of the batch does
+// not have are skipped whole.
 template <int RPT, int T>
 constexpr bool kMatrixInRegisters = RPT * T <= 2048;
 
