@@ -58,7 +58,7 @@ def test_threads_of_a_cta_agree_when_the_last_total_lands_as_time_runs_out(form)
     total first, a CTA goes on or gives up as one, and no sum that is used is wrong."""
     seen = set()
     for k in range(120):
-        got = _check(4, form, 6, 1, 2, 250 + k, 300)
+        got = _check(4, form, 6, 1, 2, 200 + 2 * k, 300)
         assert got in ([0] * 4, [TIMEOUT] * 4), (k, got)
         seen.add(got[0])
     assert seen == {0, TIMEOUT}
